@@ -1912,7 +1912,7 @@ static int run_pipeline(fnec_batch *b) {
             forked = b->side && b->ev_fork && b->ev_join && cudaEventRecord(b->ev_fork, st) == cudaSuccess &&
                      cudaStreamWaitEvent(b->side, b->ev_fork, 0) == cudaSuccess;
         }
-        launch_backsub(b->d_units, nu, b->max_s, b->d_a, b->d_x, b->d_status, forked ? b->side : st);
+        launch_backsub(b->d_units, nu, b->max_s, b->grid.d_order, b->d_a, b->d_x, b->d_status, forked ? b->side : st);
         if (b->max_rhs > 1) {
             launch_extra_rhs_exact(b->d_solves, ns, b->max_s, b->d_ants, b->d_ibuf, b->d_z, b->d_rhs, b->d_cos,
                                    b->d_a, b->d_piv, b->d_x, b->d_status, st, grouped ? b->d_rhs_groups : nullptr,

@@ -111,7 +111,7 @@ void launch_gram_exact(const UnitDesc *units, int nu, int max_w, const AntDesc *
 // returns the number of kernel launches issued
 uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const GridPlan &gp, cx *A,
                              int32_t *piv, int32_t *status, cudaStream_t st);
-void launch_backsub(const UnitDesc *units, int nu, int max_s, const cx *A, cx *x,
+void launch_backsub(const UnitDesc *units, int nu, int max_s, const int32_t *order, const cx *A, cx *x,
                     const int32_t *status, cudaStream_t st);
 // plane-wave forcing and homogeneous columns of the hom2 solves (x holds
 // the incident field until the solve overwrites it)

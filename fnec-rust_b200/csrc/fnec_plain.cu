@@ -846,95 +846,137 @@ __global__ void __launch_bounds__(256) k_trailing(const UnitDesc *__restrict__ u
 }
 
 // Back substitution x_i = (b_i - sum_{j>i} a_ij x_j) / a_ii, j ascending.
-// One warp per unit.  The subtraction chain is sequential in the reference
-// and stays sequential here; what is parallel is the memory stream.  The
-// products a_ij x_j of a 32-wide chunk are formed one per lane, every lane
-// runs the same in-order chain over the chunk through shuffles, and the U
-// entries of the next BS_DEPTH chunks (in exactly the order the chain will
-// consume them, across row boundaries) are already in flight while a chunk
-// is consumed.  b_i and a_ii are fetched one row ahead.  x lives in shared
-// memory and may alias b: b_i is read before x_i is written, and only
-// x_j, j > i, is read after.
-constexpr int BS_DEPTH = 8;
-constexpr size_t BS_SMEM_MAX = 220 * 1024;  // x staged in shared memory up to S = 14080
+// The reference's subtraction chain is sequential, and since each row's
+// first term needs the x just found, all S^2/2 subtractions form one
+// dependent chain; its bound is that count times the latency of a double
+// add.  So one warp does nothing but the chain, and two warps form the
+// products ahead of it: the U entries arrive by cp.async in pieces of BP
+// columns three pieces ahead, and the piece after the one being subtracted
+// is multiplied by its x in place.  A row's products start at column i + 2;
+// the chain warp itself forms a_{i,i+1} x_{i+1}, the only term whose x is
+// new when the row begins.  One barrier per piece.
+// Measured, 20 x 20 mesh (S = 2520, 3.2 M subtractions): 48.4 ms with one
+// warp that formed and shuffled the products between the subtractions (30
+// cycles each) -> 17.3 ms (10.6 cycles; a dependent double add takes 8.2).
+// 512 random antennas (S up to 700): 3.47 -> 1.12 ms.
+// x may alias b (b_in_x: b is read from x): b_i is read before x_i is
+// written, and only x_j, j > i, is read after.
+constexpr int BP = 256;          // products per piece: 2,000+ cycles of chain per barrier
+constexpr int BP_RING = 4;       // pieces: consumed, multiplied, two in flight
+constexpr int BP_SLOT = BP + 3;  // then a_ii, a_{i,i+1} and b_i of a row's first piece
+constexpr int BS_PROD = 64;      // product threads
+constexpr int BS_THREADS = 32 + BS_PROD;
+constexpr size_t BS_RING_BYTES = sizeof(cx) * BP_RING * BP_SLOT;
+constexpr size_t BS_SMEM_MAX = 226 * 1024;  // x staged in shared memory beside the ring up to S = 13,427
 
-struct ChunkCursor {  // (row i, first column j0) of the next 32-wide chunk
+struct PieceCursor {  // columns j0 .. j0 + BP - 1 of row i
     int i, j0;
     __device__ void next(int s) {
-        j0 += 32;
-        while (i >= 0 && j0 >= s) {
+        j0 += BP;
+        if (j0 >= s) {
             --i;
-            j0 = i + 1;
+            j0 = i + 2;
         }
     }
 };
 
-__device__ __forceinline__ cx ld_cx(const cx *p) { return *p; }
+__device__ __forceinline__ void cp_async_cx(cx *dst, const cx *src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
 
+// All BS_THREADS threads; ring: BP_RING * BP_SLOT entries of shared memory.
 __device__ __forceinline__ void backsub_rows(const cx *A, int s, int w1, const cx *bv, int64_t b_stride,
-                                             cx *s_x) {
-    int lane = threadIdx.x & 31;
-    ChunkCursor pf{s - 1, s - 32};  // positioned before the first chunk
-    pf.next(s);
-    cx u[BS_DEPTH];
-#pragma unroll
-    for (int q = 0; q < BS_DEPTH; ++q) {
-        int j = pf.j0 + lane;
-        u[q] = (pf.i >= 0 && j < s) ? A[(int64_t)pf.i * w1 + j] : cx_make(0.0, 0.0);
-        if (pf.i >= 0) pf.next(s);
+                                             bool b_in_x, cx *xs, cx *ring) {
+    const int tid = threadIdx.x, pt = tid - 32;
+    PieceCursor cur{s - 1, s + 1}, ahead = cur;
+    int t = 0;  // piece under the chain's hand
+    cx x_prev = cx_make(0.0, 0.0), sum = x_prev, diag = x_prev;
+    auto load = [&](int piece) {
+        cx *slot = ring + (piece % BP_RING) * BP_SLOT;
+        if (ahead.i >= 0) {
+            const cx *row = A + (int64_t)ahead.i * w1;
+            for (int e = pt; e < BP && ahead.j0 + e < s; e += BS_PROD) cp_async_cx(slot + e, row + ahead.j0 + e);
+            if (ahead.j0 == ahead.i + 2) {
+                if (pt == 0) cp_async_cx(slot + BP, row + ahead.i);
+                if (pt == 1 && ahead.i + 1 < s) cp_async_cx(slot + BP + 1, row + ahead.i + 1);
+                if (pt == 2 && !b_in_x) cp_async_cx(slot + BP + 2, bv + (int64_t)ahead.i * b_stride);
+            }
+            ahead.next(s);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto multiply = [&](int piece, PieceCursor c) {
+        cx *slot = ring + (piece % BP_RING) * BP_SLOT;
+        asm volatile("cp.async.wait_group 2;" ::: "memory");  // all but the two youngest pieces have landed
+        if (c.i < 0) return;
+        const int cnt = max(0, min(BP, s - c.j0)), cnt16 = (cnt + 15) & ~15;
+        // entries past the row's end are +0: sum - (+0) == sum for every sum
+        for (int e = pt; e < cnt16; e += BS_PROD)
+            slot[e] = e < cnt ? cx_mul(slot[e], xs[c.j0 + e]) : cx_make(0.0, 0.0);
+    };
+    if (tid >= 32) {
+        for (int q = 0; q < BP_RING - 1; ++q) load(q);
+        multiply(0, cur);
     }
-    cx b_next = ld_cx(bv + (int64_t)(s - 1) * b_stride);
-    cx d_next = A[(int64_t)(s - 1) * w1 + (s - 1)];
-    for (int i = s - 1; i >= 0; --i) {
-        cx sum = b_next, di = d_next;
-        if (i > 0) {
-            b_next = ld_cx(bv + (int64_t)(i - 1) * b_stride);
-            d_next = A[(int64_t)(i - 1) * w1 + (i - 1)];
-        }
-        for (int j0 = i + 1; j0 < s; j0 += 32) {
-            cx uv = u[0];
-#pragma unroll
-            for (int q = 0; q < BS_DEPTH - 1; ++q) u[q] = u[q + 1];
-            {
-                int j = pf.j0 + lane;
-                u[BS_DEPTH - 1] = (pf.i >= 0 && j < s) ? A[(int64_t)pf.i * w1 + j] : cx_make(0.0, 0.0);
-                if (pf.i >= 0) pf.next(s);
+    __syncthreads();
+    while (cur.i >= 0) {
+        if (tid >= 32) {
+            load(t + BP_RING - 1);
+            PieceCursor nx = cur;
+            nx.next(s);
+            multiply(t + 1, nx);
+        } else {
+            const cx *slot = ring + (t % BP_RING) * BP_SLOT;
+            const int cnt = (max(0, min(BP, s - cur.j0)) + 15) & ~15;
+            if (cur.j0 == cur.i + 2) {
+                diag = slot[BP];
+                sum = b_in_x ? xs[cur.i] : slot[BP + 2];
+                if (cur.i + 1 < s) sum = cx_sub(sum, cx_mul(slot[BP + 1], x_prev));
             }
-            // Lanes past the row end contribute +0: sum - (+0) == sum
-            // exactly for every sum (-0, infinities and NaN included), so
-            // the chain needs no predicate.
-            int j = j0 + lane;
-            cx p = (j < s) ? cx_mul(uv, s_x[j]) : cx_make(0.0, 0.0);
-            double pr[32], pim[32];
+            // two banks of eight products: one is read while the other is subtracted
+            cx p0[8], p1[8];
+            auto read8 = [&](cx(&p)[8], int e) {
+                const cx *q8 = slot + min(e, BP - 8);  // past the end: not used
 #pragma unroll
-            for (int q = 0; q < 32; ++q) {
-                pr[q] = __shfl_sync(0xffffffffu, p.re, q);
-                pim[q] = __shfl_sync(0xffffffffu, p.im, q);
+                for (int q = 0; q < 8; ++q) p[q] = q8[q];
+            };
+            read8(p0, 0);
+#pragma unroll 1
+            for (int e = 0; e < cnt; e += 16) {
+                read8(p1, e + 8);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) sum = cx_sub(sum, p0[q]);
+                read8(p0, e + 16);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) sum = cx_sub(sum, p1[q]);
             }
-#pragma unroll
-            for (int q = 0; q < 32; ++q) sum = cx_sub(sum, cx_make(pr[q], pim[q]));
+            if (cur.j0 + BP >= s) {
+                x_prev = cx_div(sum, diag);
+                if (tid == 0) xs[cur.i] = x_prev;
+            }
         }
-        cx xi = cx_div(sum, di);
-        __syncwarp();
-        if (lane == 0) s_x[i] = xi;
-        __syncwarp();
+        cur.next(s);
+        ++t;
+        __syncthreads();
     }
 }
 
-// staged == 0 (systems whose x does not fit in shared memory): x is built
-// in place in global memory; __syncwarp orders the warp's accesses there too.
-__global__ void k_backsub(const UnitDesc *__restrict__ units, const cx *__restrict__ abuf, cx *xbuf,
-                          const int32_t *__restrict__ status, int staged) {
+// staged == 0 (systems whose x does not fit in shared memory beside the
+// ring): x is built in place in global memory.
+__global__ void __launch_bounds__(BS_THREADS) k_backsub(const UnitDesc *__restrict__ units,
+                                                        const int32_t *__restrict__ order, const cx *__restrict__ abuf,
+                                                        cx *xbuf, const int32_t *__restrict__ status, int staged) {
     extern __shared__ cx s_xs[];
-    int ui = blockIdx.x;
+    int ui = order[blockIdx.x];  // tallest first: a tall system's chain is the batch's latency
     UnitDesc u = units[ui];
     if (status[ui] != 0) return;
     int s = u.s, w1 = s + 1;
     const cx *A = abuf + u.a_off;
-    cx *xs = staged ? s_xs : xbuf + u.x_off;
-    backsub_rows(A, s, w1, A + s, w1, xs);
+    cx *xs = staged ? s_xs + BP_RING * BP_SLOT : xbuf + u.x_off;
+    backsub_rows(A, s, w1, A + s, w1, false, xs, s_xs);
     if (staged)
-        for (int i = threadIdx.x; i < s; i += 32) xbuf[u.x_off + i] = s_xs[i];
+        for (int i = threadIdx.x; i < s; i += BS_THREADS) xbuf[u.x_off + i] = xs[i];
 }
 
 // Feedpoint rows: v_source = v_vec[idx] * dl, Zin = v_source / I[idx] when
@@ -1010,9 +1052,11 @@ __global__ void k_extra_rhs_b(const UnitDesc *__restrict__ solves, const AntDesc
     }
 }
 
-__global__ void k_extra_rhs_solve(const UnitDesc *__restrict__ solves, const cx *__restrict__ abuf,
-                                  const int32_t *__restrict__ piv_buf, cx *xbuf,
-                                  const int32_t *__restrict__ status, int staged, int first_rhs) {
+__global__ void __launch_bounds__(BS_THREADS) k_extra_rhs_solve(const UnitDesc *__restrict__ solves,
+                                                                const cx *__restrict__ abuf,
+                                                                const int32_t *__restrict__ piv_buf, cx *xbuf,
+                                                                const int32_t *__restrict__ status, int staged,
+                                                                int first_rhs) {
     extern __shared__ cx s_bs[];
     UnitDesc u = solves[blockIdx.x];
     if (u.rhs < first_rhs || status[u.sys] != 0) return;
@@ -1020,12 +1064,12 @@ __global__ void k_extra_rhs_solve(const UnitDesc *__restrict__ solves, const cx 
     const cx *A = abuf + u.a_off;
     const int32_t *piv = piv_buf + u.piv_off;
     cx *x = xbuf + u.x_off;
-    cx *s_b = staged ? s_bs : x;  // unstaged: work in place in global memory
-    int lane = threadIdx.x;
+    cx *s_b = staged ? s_bs + BP_RING * BP_SLOT : x;  // unstaged: work in place in global memory
+    const int tid = threadIdx.x;
     if (staged)
-        for (int i = lane; i < s; i += 32) s_b[i] = x[i];
-    __syncwarp();
-    if (lane == 0)
+        for (int i = tid; i < s; i += BS_THREADS) s_b[i] = x[i];
+    __syncthreads();
+    if (tid == 0)
         for (int c = 0; c < s; ++c) {
             int p = piv[c];
             if (p != c) {
@@ -1034,17 +1078,18 @@ __global__ void k_extra_rhs_solve(const UnitDesc *__restrict__ solves, const cx 
                 s_b[p] = t0;
             }
         }
-    __syncwarp();
+    __syncthreads();
     // forward: row r receives b[r] -= f[r][c] * b[c] for c = 0..r-1 in order
     for (int c = 0; c < s; ++c) {
         cx bc = s_b[c];
-        for (int r = c + 1 + lane; r < s; r += 32) s_b[r] = cx_sub(s_b[r], cx_mul(A[(int64_t)r * w1 + c], bc));
-        __syncwarp();
+        for (int r = c + 1 + tid; r < s; r += BS_THREADS)
+            s_b[r] = cx_sub(s_b[r], cx_mul(A[(int64_t)r * w1 + c], bc));
+        __syncthreads();
     }
     // back substitution, j ascending, as k_backsub (x overwrites b in place)
-    backsub_rows(A, s, w1, s_b, 1, s_b);
+    backsub_rows(A, s, w1, s_b, 1, true, s_b, s_bs);
     if (staged)
-        for (int i = lane; i < s; i += 32) x[i] = s_b[i];
+        for (int i = tid; i < s; i += BS_THREADS) x[i] = s_b[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -1061,6 +1106,7 @@ __global__ void k_extra_rhs_solve(const UnitDesc *__restrict__ solves, const cx 
 // ---------------------------------------------------------------------------
 constexpr int RG = 32;  // solves per group
 constexpr int SG = 16;  // solves per substitution block: a [s][16] tile, several blocks per SM
+constexpr size_t GS_SMEM_MAX = 220 * 1024;  // their dynamic shared memory
 
 __global__ void __launch_bounds__(64) k_extra_rhs_b_group(const UnitDesc *__restrict__ solves,
                                                           const int4 *__restrict__ groups,
@@ -1546,16 +1592,25 @@ uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const Gri
     }
     return L;
 }
-void launch_backsub(const UnitDesc *units, int nu, int max_s, const cx *A, cx *x,
-                    const int32_t *status, cudaStream_t st) {
-    size_t smem = sizeof(cx) * (size_t)max_s;
-    int staged = smem <= BS_SMEM_MAX;
-    if (staged && smem > 0) {  // static + dynamic above 48 KB needs the raised limit
-        int lim = set_smem_limit_once(k_backsub, (int)BS_SMEM_MAX);
-        if (lim < 0 || (size_t)lim < smem) staged = 0;
+// Dynamic shared memory of the chain kernels for systems of up to max_s
+// unknowns: the product ring, and x beside it (*staged) where both fit.
+template <typename K>
+static size_t backsub_smem(K kernel, int max_s, int *staged) {
+    const size_t smem = BS_RING_BYTES + sizeof(cx) * (size_t)max_s;
+    *staged = smem <= BS_SMEM_MAX;
+    if (*staged) {  // static + dynamic above 48 KB needs the raised limit
+        int lim = set_smem_limit_once(kernel, (int)BS_SMEM_MAX);
+        if (lim < 0 || (size_t)lim < smem) *staged = 0;
     }
-    if (!staged) smem = 0;
-    if (nu > 0) k_backsub<<<nu, 32, smem, st>>>(units, A, x, status, staged);
+    return *staged ? smem : BS_RING_BYTES;
+}
+
+void launch_backsub(const UnitDesc *units, int nu, int max_s, const int32_t *order, const cx *A, cx *x,
+                    const int32_t *status, cudaStream_t st) {
+    if (nu <= 0) return;
+    int staged = 0;
+    const size_t smem = backsub_smem(k_backsub, max_s, &staged);
+    k_backsub<<<nu, BS_THREADS, smem, st>>>(units, order, A, x, status, staged);
 }
 // matrix.rs:131-139 add_to_diagonal / add_to_entry: each stamp one
 // separately rounded complex add, an entry's stamps in their order (the
@@ -1586,33 +1641,28 @@ void launch_extra_rhs_exact(const UnitDesc *solves, int ns, int max_s, const Ant
         dim3 gb((max_s + 63) / 64, n_groups);
         k_extra_rhs_b_group<<<gb, 64, 0, st>>>(solves, groups, ants, ibuf, z, rhs, cosv, x);
         const size_t smem4 = solve_group4_smem(max_s);
-        int lim4 = (smem4 <= BS_SMEM_MAX && max_s <= RB * GW4 * 32)
-                       ? set_smem_limit_once(k_extra_rhs_solve_group4, (int)BS_SMEM_MAX)
+        int lim4 = (smem4 <= GS_SMEM_MAX && max_s <= RB * GW4 * 32)
+                       ? set_smem_limit_once(k_extra_rhs_solve_group4, (int)GS_SMEM_MAX)
                        : -1;
         if (lim4 >= 0 && (size_t)lim4 >= smem4) {
             k_extra_rhs_solve_group4<<<n_groups, GW4 * 32, smem4, st>>>(solves, groups, A, piv, x, status);
             return;
         }
         const size_t smem = (sizeof(cx) * (SG + 1) + sizeof(int32_t)) * (size_t)max_s;
-        int lim = smem <= BS_SMEM_MAX ? set_smem_limit_once(k_extra_rhs_solve_group, (int)BS_SMEM_MAX) : -1;
+        int lim = smem <= GS_SMEM_MAX ? set_smem_limit_once(k_extra_rhs_solve_group, (int)GS_SMEM_MAX) : -1;
         if (lim >= 0 && (size_t)lim >= smem) {
             k_extra_rhs_solve_group<<<dim3(n_groups, RG / SG), SG, smem, st>>>(solves, groups, A, piv, x, status);
             return;
         }
-        // a factor too tall for the shared tile: one warp per solve on the b vectors formed above
-        k_extra_rhs_solve<<<ns, 32, 0, st>>>(solves, A, piv, x, status, 0, 1);
+        // a factor too tall for the shared tile: one block per solve on the b vectors formed above
+        k_extra_rhs_solve<<<ns, BS_THREADS, BS_RING_BYTES, st>>>(solves, A, piv, x, status, 0, 1);
         return;
     }
     dim3 g((max_s + 127) / 128, ns);
     k_extra_rhs_b<<<g, 128, 0, st>>>(solves, ants, ibuf, z, rhs, cosv, x, first_rhs);
-    size_t smem = sizeof(cx) * (size_t)max_s;
-    int staged = smem <= BS_SMEM_MAX;
-    if (staged && smem > 0) {  // static + dynamic above 48 KB needs the raised limit
-        int lim = set_smem_limit_once(k_extra_rhs_solve, (int)BS_SMEM_MAX);
-        if (lim < 0 || (size_t)lim < smem) staged = 0;
-    }
-    if (!staged) smem = 0;
-    k_extra_rhs_solve<<<ns, 32, smem, st>>>(solves, A, piv, x, status, staged, first_rhs);
+    int staged = 0;
+    const size_t smem = backsub_smem(k_extra_rhs_solve, max_s, &staged);
+    k_extra_rhs_solve<<<ns, BS_THREADS, smem, st>>>(solves, A, piv, x, status, staged, first_rhs);
 }
 
 }  // namespace fnec
