@@ -52,16 +52,18 @@
 
 #ifdef __CUDACC__
 #define FNEC_LIBM_FN __host__ __device__ __forceinline__
+#define FNEC_LIBM_MEMBER __host__ __device__ __forceinline__
 #else
 #define FNEC_LIBM_FN static inline
+#define FNEC_LIBM_MEMBER inline
 #endif
 
 namespace fnec_libm {
 
 // sin(i/128) hi, lo, cos(i/128) hi, lo for i = 0..109.  The device copy
-// lives in global memory and is read through the read-only cache: the lanes
-// of a warp index it with different points, which the constant cache would
-// serialise.
+// lives in global memory, not in the constant cache: the lanes of a warp
+// index it with different points.  Kernels that are bound by these reads
+// stage it in shared memory (Z fill, fnec_plain.cu).
 #ifdef __CUDACC__
 static __device__ const double libm_sincos_tab_dev[440] = {
 #include "libm_tables.inc"
@@ -106,28 +108,46 @@ FNEC_LIBM_FN double lm_copysign(double a, double b) {
 #endif
 }
 
+// The coefficients and splits below, in the constant bank on the device: a
+// double whose low word is not zero does not fit an instruction, and as a
+// literal takes two moves into registers at every use (with 64 registers a
+// thread they were a fifth of the fill's instructions).
+#ifdef __CUDACC__
+static __constant__ double lm_const_dev[16] = {
+    -0.16666666666666666, 0.0083333333333323288, -0.00019841269834414642,
+    2.755729806860771e-06, -2.5022014848318398e-08, -1.66666666666664880952546298448555E-01,
+    8.33333214285722277379541354343671E-03, -4.16666666666664434524222570944589E-02, 1.38888874007937613028114285595617E-03,
+    0x1.921fb54442d18p+0, 0x1.1a62633145c07p-54, 0x1.921fb58p+0,
+    -0x1.dde973cp-27, -0x1.cb3b398p-55, -0x1.d747f23e32ed7p-83,
+    0x1.45f306dc9c883p-1};
+#endif
+#ifdef __CUDA_ARCH__
+#define LM_K(i, v) lm_const_dev[i]
+#else
+#define LM_K(i, v) (v)
+#endif
 // polynomial coefficients (usncs.h)
-#define LM_S1 (-0.16666666666666666)
-#define LM_S2 0.0083333333333323288
-#define LM_S3 (-0.00019841269834414642)
-#define LM_S4 2.755729806860771e-06
-#define LM_S5 (-2.5022014848318398e-08)
-#define LM_SN3 (-1.66666666666664880952546298448555E-01)
-#define LM_SN5 8.33333214285722277379541354343671E-03
+#define LM_S1 LM_K(0, -0.16666666666666666)
+#define LM_S2 LM_K(1, 0.0083333333333323288)
+#define LM_S3 LM_K(2, -0.00019841269834414642)
+#define LM_S4 LM_K(3, 2.755729806860771e-06)
+#define LM_S5 LM_K(4, -2.5022014848318398e-08)
+#define LM_SN3 LM_K(5, -1.66666666666664880952546298448555E-01)
+#define LM_SN5 LM_K(6, 8.33333214285722277379541354343671E-03)
 #define LM_CS2 4.99999999999999999999950396842453E-01
-#define LM_CS4 (-4.16666666666664434524222570944589E-02)
-#define LM_CS6 1.38888874007937613028114285595617E-03
+#define LM_CS4 LM_K(7, -4.16666666666664434524222570944589E-02)
+#define LM_CS6 LM_K(8, 1.38888874007937613028114285595617E-03)
 // 1.5 * 2^45: adding it rounds to a multiple of 1/128
 #define LM_BIG 52776558133248.0
 // pi/2 = hp0 + hp1
-#define LM_HP0 0x1.921fb54442d18p+0
-#define LM_HP1 0x1.1a62633145c07p-54
+#define LM_HP0 LM_K(9, 0x1.921fb54442d18p+0)
+#define LM_HP1 LM_K(10, 0x1.1a62633145c07p-54)
 // pi/2 = mp1 + mp2 + pp3 + pp4 (mp1, mp2 short enough for exact n * mp)
-#define LM_MP1 0x1.921fb58p+0
-#define LM_MP2 (-0x1.dde973cp-27)
-#define LM_PP3 (-0x1.cb3b398p-55)
-#define LM_PP4 (-0x1.d747f23e32ed7p-83)
-#define LM_HPINV 0x1.45f306dc9c883p-1
+#define LM_MP1 LM_K(11, 0x1.921fb58p+0)
+#define LM_MP2 LM_K(12, -0x1.dde973cp-27)
+#define LM_PP3 LM_K(13, -0x1.cb3b398p-55)
+#define LM_PP4 LM_K(14, -0x1.d747f23e32ed7p-83)
+#define LM_HPINV LM_K(15, 0x1.45f306dc9c883p-1)
 #define LM_TOINT 6755399441055744.0
 
 // sin(a + da) for |a| < 0.126: odd Taylor polynomial
@@ -233,49 +253,103 @@ FNEC_LIBM_FN double libm_cos(double x) {
     return x - x + NAN;
 }
 
-// (libm_sin(x), libm_cos(x)) with the branch and the reduction shared:
-// glibc's sincos returns the same two values as sin and cos.  Every branch
-// evaluates one do_sin and one do_cos; only their arguments differ, so the
-// branch picks arguments and the two evaluations run once for all lanes of
-// a warp whose arguments fall in different branches.
-FNEC_LIBM_FN void libm_sincos(double x, double *s, double *c) {
-    uint32_t k = (uint32_t)(lm_bits(x) >> 32) & 0x7fffffffu;
-    double as, das, ac, dac;
-    int mode, n = 0;
-    if (k < 0x3feb6000u) {  // |x| < 0.855469: the table around x itself
-        as = ac = x;
-        das = dac = 0.0;
-        mode = 0;
-    } else if (k < 0x400368fdu) {  // |x| < 2.426265: taken from pi/2
-        double y = LM_SUB(LM_HP0, fabs(x));
-        ac = y;  // sin x = copysign(cos(y + hp1), x)
-        dac = LM_HP1;
-        as = LM_ADD(y, LM_HP1);  // cos x = sin(a + da)
-        das = LM_ADD(LM_SUB(y, as), LM_HP1);
-        mode = 1;
-    } else if (k < 0x419921fbu) {  // x - n pi/2
-        double a, da;
-        n = lm_reduce(x, &a, &da);
-        as = ac = a;
-        das = dac = da;
-        mode = 2;
-    } else {
-        *s = *c = x - x + NAN;
+// One point of the table: sin and cos of i/128 in two parts each.
+struct LmEntry {
+    double sn, ssn, cs, ccs;
+};
+// The table in global memory (the host's array in a host build).
+struct LmTable {
+    FNEC_LIBM_MEMBER LmEntry operator()(int i) const {
+        return {LM_TAB(4 * i), LM_TAB(4 * i + 1), LM_TAB(4 * i + 2), LM_TAB(4 * i + 3)};
+    }
+};
+
+// a with its sign bit turned where m's is set (m: a high word)
+FNEC_LIBM_FN double lm_turn(double a, uint32_t m) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double(__double2hiint(a) ^ (int)(m & 0x80000000u), __double2loint(a));
+#else
+    uint64_t u = lm_bits(a) ^ ((uint64_t)(m & 0x80000000u) << 32);
+    double r;
+    memcpy(&r, &u, 8);
+    return r;
+#endif
+}
+FNEC_LIBM_FN uint32_t lm_hi(double a) { return (uint32_t)(lm_bits(a) >> 32); }
+
+// lm_do_cos with the table point given: u = LM_BIG + |x|
+FNEC_LIBM_FN double lm_cos_at(double x, double dx, double u, const LmEntry &e) {
+    const double r = LM_ADD(LM_SUB(fabs(x), LM_SUB(u, LM_BIG)), lm_turn(dx, lm_hi(x)));
+    const double xx = LM_MUL(r, r);
+    const double t = LM_FMA(LM_MUL(r, xx), LM_FMA(xx, LM_SN5, LM_SN3), r);
+    const double v = LM_MUL(xx, LM_FMA(xx, LM_FMA(xx, LM_CS6, LM_CS4), LM_CS2));
+    double cor = LM_FMA(-t, e.ssn, e.ccs);
+    cor = LM_FMA(-e.cs, v, cor);
+    cor = LM_FMA(-e.sn, t, cor);
+    return LM_ADD(e.cs, cor);
+}
+// lm_do_sin with the table point given: both its forms, the Taylor one
+// selected below 0.126
+FNEC_LIBM_FN double lm_sin_at(double x, double dx, double u, const LmEntry &e) {
+    const double d = lm_turn(dx, lm_hi(x));
+    const double r = LM_SUB(fabs(x), LM_SUB(u, LM_BIG));
+    const double xx = LM_MUL(r, r);
+    const double t = LM_ADD(r, LM_FMA(LM_MUL(r, xx), LM_FMA(xx, LM_SN5, LM_SN3), d));
+    const double v = LM_FMA(r, d, LM_MUL(xx, LM_FMA(xx, LM_FMA(xx, LM_CS6, LM_CS4), LM_CS2)));
+    double cor = LM_FMA(t, e.ccs, e.ssn);
+    cor = LM_FMA(-e.sn, v, cor);
+    cor = LM_FMA(e.cs, t, cor);
+    const double far = lm_turn(LM_ADD(e.sn, cor), lm_hi(x));
+    const double near = lm_taylor_sin(LM_MUL(x, x), x, dx);
+    return (lm_bits(x) & 0x7fffffffffffffffull) < 0x3fc020c49ba5e354ull ? near : far;  // |x| < 0.126
+}
+
+// (libm_sin(x), libm_cos(x)): glibc's sincos returns the same two values as
+// sin and cos.  Every branch of the two evaluates one do_sin and one do_cos
+// whose arguments differ from each other by the 6e-17 of hp1 at most, so
+// the branch only picks the arguments, and both are evaluated straight
+// through from one table entry (tab(i); a second one in the rare case that
+// the two arguments round to different points): a warp's lanes hold
+// arguments of every branch.
+template <class Tab>
+FNEC_LIBM_FN void libm_sincos(double x, double *s, double *c, const Tab &tab) {
+    const uint32_t hi = lm_hi(x), k = hi & 0x7fffffffu;
+    if (k - 0x3e400000u >= 0x419921fbu - 0x3e400000u) {
+        if (k < 0x3e400000u) {  // |x| < 2^-27
+            *s = x;
+            *c = 1.0;
+        } else {  // outside the restated range (or inf/nan)
+            *s = *c = x - x + NAN;
+        }
         return;
     }
-    const double sp = lm_do_sin(as, das), cp = lm_do_cos(ac, dac);
-    if (mode == 0) {
-        *s = k < 0x3e500000u ? x : sp;
-        *c = k < 0x3e400000u ? 1.0 : cp;
-    } else if (mode == 1) {
-        *s = lm_copysign(cp, x);
-        *c = sp;
-    } else {
-        double sv = (n & 1) ? cp : sp, cv = (n & 1) ? sp : cp;
-        *s = (n & 2) ? -sv : sv;
-        *c = ((n + 1) & 2) ? -cv : cv;
+    double as = x, das = 0.0, ac = x, dac = 0.0;
+    int n = 0;               // the quadrant; 0 below 0.855469: the table around x itself
+    if (k >= 0x400368fdu) {  // |x| >= 2.426265: x - n pi/2
+        n = lm_reduce(x, &as, &das);
+        ac = as;
+        dac = das;
+    } else if (k >= 0x3feb6000u) {  // taken from pi/2, with y = hp0 - |x|
+        n = hi >> 31 ? 3 : 1;       // sin x = copysign(cos(y + hp1), x), cos x = sin(a + da)
+        ac = LM_SUB(LM_HP0, fabs(x));
+        dac = LM_HP1;
+        as = LM_ADD(ac, LM_HP1);
+        das = LM_ADD(LM_SUB(ac, as), LM_HP1);
+        if (n == 1) {  // cos x = -sin(-(a + da))
+            as = -as;
+            das = -das;
+        }
     }
+    const double us = LM_ADD(LM_BIG, fabs(as)), uc = LM_ADD(LM_BIG, fabs(ac));
+    const int is = (int)(lm_bits(us) & 0xffffffffu), ic = (int)(lm_bits(uc) & 0xffffffffu);
+    const LmEntry e = tab(is);
+    const double sp = lm_sin_at(as, das, us, e);
+    double cp = lm_cos_at(ac, dac, uc, e);
+    if (ic != is) cp = lm_cos_at(ac, dac, uc, tab(ic));
+    *s = lm_turn((n & 1) ? cp : sp, (uint32_t)n << 30);
+    *c = lm_turn((n & 1) ? sp : cp, (uint32_t)(n + 1) << 30);
 }
+FNEC_LIBM_FN void libm_sincos(double x, double *s, double *c) { libm_sincos(x, s, c, LmTable{}); }
 
 // f64::hypot on linux-gnu: glibc 2.35+ sysdeps/ieee754/dbl-64/e_hypot.c
 // (Borges, "An Improved Algorithm for hypot(a, b)", the variant without

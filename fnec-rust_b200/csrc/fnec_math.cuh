@@ -22,6 +22,7 @@
 #define D_MUL(a, b) __dmul_rn((a), (b))
 #define D_DIV(a, b) __ddiv_rn((a), (b))
 #define D_SQRT(a) __dsqrt_rn((a))
+#define D_FMA(a, b, c) __fma_rn((a), (b), (c))
 #else
 #define FNEC_FN static inline
 #define D_ADD(a, b) ((a) + (b))
@@ -29,6 +30,7 @@
 #define D_MUL(a, b) ((a) * (b))
 #define D_DIV(a, b) ((a) / (b))
 #define D_SQRT(a) sqrt((a))
+#define D_FMA(a, b, c) fma((a), (b), (c))
 #endif
 
 namespace fnec {
@@ -61,5 +63,53 @@ FNEC_FN cx cx_div(cx a, cx b) {
 // Complex64::norm = f64::hypot, as the platform libm evaluates it
 FNEC_FN double cx_norm(cx a) { return fnec_libm::libm_hypot(a.re, a.im); }
 FNEC_FN double cx_norm_sqr(cx a) { return D_ADD(D_MUL(a.re, a.re), D_MUL(a.im, a.im)); }
+
+// ---------------------------------------------------------------------------
+// Correctly rounded sqrt(x) and quotients by it, from one reciprocal square
+// root: the fill's G(R) takes a square root and two divisions by it, and the
+// three together cost less than one general division here.
+//   y  = 1/sqrt(x): a single-precision first guess y0, then Householder's
+//        cubic step y0 (1 + e/2 + 3 e^2/8) with e = 1 - x y0^2 (|e| < 2^-21,
+//        so the step leaves 2^-65 beside the roundings);
+//   r  = g + (x - g^2) y/2 with g = x y, the residual exact in an FMA;
+//   z  = y + y (1 - r y), the reciprocal of r;
+//   a/r = q + (a - q r) z with q = a z.
+// The last two corrections are Markstein's (Computation of elementary
+// functions on the IBM RISC System/6000 processor, 1990): the value before
+// the final rounding is within 2^-103 of exact, relative, and the result is
+// the rounded one.  Domain: x normal in [2^-100, 2^100) and quotients whose
+// residual stays normal (a zero, or |a| above 2^-800); callers fall back to
+// the general operations outside.
+// ---------------------------------------------------------------------------
+struct SqrtRecip {
+    double r, z;  // sqrt(x), 1/sqrt(x) rounded from r
+};
+FNEC_FN SqrtRecip sqrt_recip(double x) {
+#ifdef __CUDA_ARCH__
+    float f;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(__double2float_rn(x)));
+    const double y0 = (double)f;
+#else
+    const double y0 = (double)(1.0f / sqrtf((float)x));
+#endif
+    const double e = D_FMA(-D_MUL(x, y0), y0, 1.0);
+    const double y = D_FMA(D_MUL(y0, e), D_FMA(e, 0.375, 0.5), y0);
+    const double g = D_MUL(x, y);
+    const double r = D_FMA(D_FMA(-g, g, x), D_MUL(0.5, y), g);
+    double z = D_FMA(D_FMA(-r, y, 1.0), y, y);
+    // an all-ones mantissa is the one whose reciprocal that step can leave
+    // an ulp off (1/r lies just above the middle of two doubles)
+    if ((uint32_t)fnec_libm::lm_bits(r) == 0xffffffffu) z = D_DIV(1.0, r);
+    return {r, z};
+}
+// a / sr.r (the residual with its sign turned twice: a zero keeps its sign)
+FNEC_FN double div_by(double a, SqrtRecip sr) {
+    const double q = D_MUL(a, sr.z);
+    return D_FMA(-D_FMA(q, sr.r, -a), sr.z, q);
+}
+FNEC_FN bool sqrt_recip_domain(double x) {
+    const uint32_t k = (uint32_t)(fnec_libm::lm_bits(x) >> 32);
+    return k - 0x39b00000u < 0x46300000u - 0x39b00000u;  // 2^-100 <= x < 2^100
+}
 
 }  // namespace fnec

@@ -270,94 +270,146 @@ __device__ __forceinline__ cx green_k_exact(double r, double k) {
     return cx_make(D_DIV(cs, r), D_DIV(sn, r));
 }
 
-// matrix.rs:297-331 elem(obs, src, k, is_self); self_log is the source
-// segment's 2 ln((h + sqrt(h^2 + a^2)) / a), evaluated on the host
-__device__ __forceinline__ cx elem_exact(const double *om, const double *od, const double *sm,
-                                         const double *sd, double slen, double srad, double self_log, double k,
-                                         bool is_self) {
-    double cos_alpha = D_ADD(D_ADD(D_MUL(od[0], sd[0]), D_MUL(od[1], sd[1])), D_MUL(od[2], sd[2]));
-    double half = D_MUL(slen, 0.5);
-    double a = srad;
-    double ire, iim;
-    if (is_self) {
-        double sre = 0.0, sim = 0.0;
-#pragma unroll 1
-        for (int m = 0; m < 4; ++m) {
-            double l = D_MUL(c_gl_n4[m], half);
-            double r_eff = D_SQRT(D_ADD(D_MUL(l, l), D_MUL(a, a)));
-            cx g = green_k_exact(r_eff, k);
-            double dre = D_SUB(g.re, D_DIV(1.0, r_eff));
-            sre = D_ADD(sre, D_MUL(c_gl_w4[m], dre));
-            sim = D_ADD(sim, D_MUL(c_gl_w4[m], g.im));
-        }
-        sre = D_MUL(sre, half);
-        sim = D_MUL(sim, half);
-        ire = D_ADD(sre, self_log);
-        iim = sim;
-    } else {
-        double sre = 0.0, sim = 0.0;
-#pragma unroll 1
-        for (int m = 0; m < 8; ++m) {
-            double sc = D_MUL(c_gl_n8[m], half);
-            double rs0 = D_ADD(sm[0], D_MUL(sc, sd[0]));
-            double rs1 = D_ADD(sm[1], D_MUL(sc, sd[1]));
-            double rs2 = D_ADD(sm[2], D_MUL(sc, sd[2]));
-            double r0 = D_SUB(om[0], rs0), r1 = D_SUB(om[1], rs1), r2 = D_SUB(om[2], rs2);
-            double r_sq = D_ADD(D_ADD(D_MUL(r0, r0), D_MUL(r1, r1)), D_MUL(r2, r2));
-            double r_eff = D_SQRT(D_ADD(r_sq, D_MUL(a, a)));
-            cx g = green_k_exact(r_eff, k);
-            sre = D_ADD(sre, D_MUL(c_gl_w8[m], g.re));
-            sim = D_ADD(sim, D_MUL(c_gl_w8[m], g.im));
-        }
-        ire = D_MUL(sre, half);
-        iim = D_MUL(sim, half);
+// The fill of a 16 x 16 tile by 256 threads.  What bounds it is the FP64
+// pipe (about 85 operations a sample) once the rest keeps out of its way:
+// - the sin/cos table sits in shared memory as four arrays (the lanes look
+//   up different points; from global memory those scattered reads took
+//   three quarters of the kernel's time, 30 % FP64 pipe);
+// - a sample's source point mid + node * half * dir depends on (source,
+//   node) alone and is formed once per tile.  The PEC image's points are the
+//   direct ones of the mirrored node with z negated: the nodes are symmetric
+//   and a rounded sum with both signs turned is the same sum turned;
+// - the square root and the two divisions of G(R) share one reciprocal
+//   square root (sqrt_recip).
+// Two nodes in flight per thread at 4 CTAs per SM (one: 4.50 ms, 2 CTAs with
+// 128 registers: 5.2 ms).  Measured, 512 random antennas: 9.26 -> 4.36 ms,
+// FP64 pipe 30 -> 57 %; the rest is issue slots of the branches and selects.
+struct FillTile {
+    double tab[4][112];     // the sin/cos table by part
+    double rs[8][3][16];    // source points (node, axis, source)
+    double om[3][16], od[3][16], sd[3][16];
+    double half[16], a2[16], rad[16], self_log[16];
+};
+
+struct LmSharedTable {
+    const double (*t)[112];
+    __device__ __forceinline__ fnec_libm::LmEntry operator()(int i) const {
+        return {t[0][i], t[1][i], t[2][i], t[3][i]};
     }
-    return cx_make(D_MUL(ire, cos_alpha), D_MUL(iim, cos_alpha));
+};
+
+// w G(R) at R^2 = x added to the sums
+__device__ __forceinline__ void add_green(double x, double k, double w, const LmSharedTable &tab, double &sre,
+                                          double &sim) {
+    double gr, gi, sn, cs;
+    SqrtRecip sr = sqrt_recip(x);
+    double t = D_MUL(-k, sr.r);
+    const uint32_t kt = (uint32_t)(fnec_libm::lm_bits(t) >> 32) & 0x7fffffffu;
+    if (sqrt_recip_domain(x) && kt >= 0x39b00000u) {  // kR at least 2^-100: its sine's quotient stays normal
+        fnec_libm::libm_sincos(t, &sn, &cs, tab);
+        gr = div_by(cs, sr);
+        gi = div_by(sn, sr);
+    } else {
+        const cx g = green_k_exact(D_SQRT(x), k);
+        gr = g.re;
+        gi = g.im;
+    }
+    sre = D_ADD(sre, D_MUL(w, gr));
+    sim = D_ADD(sim, D_MUL(w, gi));
 }
 
-__device__ __forceinline__ cx z_entry_exact(const DevSeg &o, const DevSeg &s, double k, int ground,
-                                            bool is_self) {
-    cx direct = elem_exact(o.mid, o.dir, s.mid, s.dir, s.len, s.rad, s.self_log, k, is_self);
-    cx img = cx_make(0.0, 0.0);
-    if (ground == 1) {
-        // matrix.rs:265-279 image: position (x, y, -z), current (-Jx, -Jy, +Jz)
-        double im_mid[3] = {s.mid[0], s.mid[1], -s.mid[2]};
-        double im_dir[3] = {-s.dir[0], -s.dir[1], s.dir[2]};
-        img = elem_exact(o.mid, o.dir, im_mid, im_dir, s.len, s.rad, 0.0, k, false);
+// matrix.rs:186-218: Z[i][j] for rows row0.. and columns col0.. of one system
+__device__ __forceinline__ void fill_exact_tile(FillTile &sh, const DevSeg *__restrict__ sg, int n, double k,
+                                                int ground, int row0, int col0, cx *__restrict__ z) {
+    const int tid = threadIdx.x;
+    for (int e = tid; e < 440; e += 256) sh.tab[e & 3][e >> 2] = __ldg(&fnec_libm::libm_sincos_tab_dev[e]);
+    if (tid < 128) {  // (source, node)
+        const int j = min(col0 + (tid & 15), n - 1), m = tid >> 4;
+        const DevSeg &s = sg[j];
+        const double half = D_MUL(s.len, 0.5), sc = D_MUL(c_gl_n8[m], half);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sh.rs[m][c][tid & 15] = D_ADD(s.mid[c], D_MUL(sc, s.dir[c]));
+        if (m == 0) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sh.sd[c][tid] = s.dir[c];
+            sh.half[tid] = half;
+            sh.rad[tid] = s.rad;
+            sh.a2[tid] = D_MUL(s.rad, s.rad);
+            sh.self_log[tid] = s.self_log;
+        }
+    } else if (tid < 144) {
+        const int i = min(row0 + tid - 128, n - 1);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sh.om[c][tid - 128] = sg[i].mid[c];
+            sh.od[c][tid - 128] = sg[i].dir[c];
+        }
     }
-    return cx_add(direct, img);
+    __syncthreads();
+    const int ii = tid >> 4, jj = tid & 15;
+    const int i = row0 + ii, j = col0 + jj;
+    if (i >= n || j >= n) return;
+    const LmSharedTable tab{sh.tab};
+    const double o0 = sh.om[0][ii], o1 = sh.om[1][ii], o2 = sh.om[2][ii];
+    const double half = sh.half[jj], a2 = sh.a2[jj];
+    cx direct = cx_make(0.0, 0.0), img = cx_make(0.0, 0.0);
+#pragma unroll 1
+    for (int image = 0; image <= (ground == 1 ? 1 : 0); ++image) {
+        // matrix.rs:297-331 elem; image (:265-279): position (x, y, -z), current (-Jx, -Jy, +Jz)
+        double sre = 0.0, sim = 0.0;
+        if (i == j && !image) {
+#pragma unroll 1
+            for (int m = 0; m < 4; ++m) {
+                double l = D_MUL(c_gl_n4[m], half);
+                double r_eff = D_SQRT(D_ADD(D_MUL(l, l), a2));
+                cx g = green_k_exact(r_eff, k);
+                sre = D_ADD(sre, D_MUL(c_gl_w4[m], D_SUB(g.re, D_DIV(1.0, r_eff))));
+                sim = D_ADD(sim, D_MUL(c_gl_w4[m], g.im));
+            }
+            sre = D_ADD(D_MUL(sre, half), sh.self_log[jj]);
+            sim = D_MUL(sim, half);
+        } else {
+            const int flip = image ? 7 : 0;
+            const uint32_t turn = image ? 0x80000000u : 0u;
+#pragma unroll 2
+            for (int m = 0; m < 8; ++m) {
+                const double(*p)[16] = sh.rs[m ^ flip];
+                const double r0 = D_SUB(o0, p[0][jj]), r1 = D_SUB(o1, p[1][jj]);
+                const double r2 = D_SUB(o2, fnec_libm::lm_turn(p[2][jj], turn));
+                const double r_sq = D_ADD(D_ADD(D_MUL(r0, r0), D_MUL(r1, r1)), D_MUL(r2, r2));
+                add_green(D_ADD(r_sq, a2), k, c_gl_w8[m], tab, sre, sim);
+            }
+            sre = D_MUL(sre, half);
+            sim = D_MUL(sim, half);
+        }
+        const double d0 = sh.sd[0][jj], d1 = sh.sd[1][jj];
+        const double cos_alpha = D_ADD(D_ADD(D_MUL(sh.od[0][ii], image ? -d0 : d0),
+                                             D_MUL(sh.od[1][ii], image ? -d1 : d1)),
+                                       D_MUL(sh.od[2][ii], sh.sd[2][jj]));
+        const cx v = cx_make(D_MUL(sre, cos_alpha), D_MUL(sim, cos_alpha));
+        if (image) img = v;
+        else direct = v;
+    }
+    z[(int64_t)i * n + j] = cx_add(direct, img);
 }
 
 // One CTA of 256 threads fills a 16x16 tile of one unit's Z.
-__global__ void __launch_bounds__(256) k_fill_exact(const UnitDesc *__restrict__ units,
-                                                    const AntDesc *__restrict__ ants,
-                                                    const DevSeg *__restrict__ segs,
-                                                    const int4 *__restrict__ tiles, cx *zbuf) {
-    __shared__ DevSeg s_obs[16];
-    __shared__ DevSeg s_src[16];
-    int4 t = tiles[blockIdx.x];  // (unit, row0, col0, -)
-    UnitDesc u = units[t.x];
-    AntDesc a = ants[u.ant];
-    int n = a.n;
-    const DevSeg *sg = segs + a.seg_off;
-    int tid = threadIdx.x;
-    if (tid < 16 && t.y + tid < n) s_obs[tid] = sg[t.y + tid];
-    if (tid >= 32 && tid < 48 && t.z + tid - 32 < n) s_src[tid - 32] = sg[t.z + tid - 32];
-    __syncthreads();
-    int ii = tid / 16, jj = tid % 16;
-    int i = t.y + ii, j = t.z + jj;
-    if (i >= n || j >= n) return;
-    cx z = z_entry_exact(s_obs[ii], s_src[jj], u.k_fill, a.ground, i == j);
-    zbuf[u.z_off + (int64_t)i * n + j] = z;
+__global__ void __launch_bounds__(256, 4) k_fill_exact(const UnitDesc *__restrict__ units,
+                                                       const AntDesc *__restrict__ ants,
+                                                       const DevSeg *__restrict__ segs,
+                                                       const int4 *__restrict__ tiles, cx *zbuf) {
+    __shared__ FillTile sh;
+    const int4 t = tiles[blockIdx.x];  // (unit, row0, col0, -)
+    const UnitDesc &u = units[t.x];
+    const AntDesc &a = ants[u.ant];
+    fill_exact_tile(sh, segs + a.seg_off, a.n, u.k_fill, a.ground, t.y, t.z, zbuf + u.z_off);
 }
 
 // Fill for caller-provided segments (ZSegmentInput): same arithmetic.
-__global__ void __launch_bounds__(256) k_fill_exact_flat(const DevSeg *__restrict__ sg, int n,
-                                                         double k, int ground, cx *z) {
-    int i = blockIdx.y * 16 + threadIdx.x / 16;
-    int j = blockIdx.x * 16 + threadIdx.x % 16;
-    if (i >= n || j >= n) return;
-    z[(int64_t)i * n + j] = z_entry_exact(sg[i], sg[j], k, ground, i == j);
+__global__ void __launch_bounds__(256, 4) k_fill_exact_flat(const DevSeg *__restrict__ sg, int n,
+                                                            double k, int ground, cx *z) {
+    __shared__ FillTile sh;
+    fill_exact_tile(sh, sg, n, k, ground, blockIdx.y * 16, blockIdx.x * 16, z);
 }
 
 // ---------------------------------------------------------------------------
