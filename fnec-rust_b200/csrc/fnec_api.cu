@@ -1286,8 +1286,13 @@ static int build_batch(fnec_ctx *ctx, std::vector<HostAnt> &hs, int precision, f
                 const int nt = (n + 15) / 16;
                 b->fill_units.push_back(make_int4(uidx, nt, (int)b->n_fill, 0));
                 b->n_fill += (int64_t)nt * nt;
-                for (int i0 = 0; i0 < n; i0 += 64)
-                    for (int j0 = 0; j0 <= n; j0 += 64) b->gram_tiles.push_back(make_int4(uidx, i0, j0, 0));
+                // Gram output tiles: the plain form's on and above the diagonal
+                // (right-hand-side column included), the mixed SIMT form's all
+                const bool plain = b->precision == FNEC_PRECISION_FP64;
+                const int gt = plain ? GRAM_TILE : 64;
+                for (int i0 = 0; i0 < n; i0 += gt)
+                    for (int j0 = plain ? i0 : 0; j0 <= n; j0 += gt)
+                        b->gram_tiles.push_back(make_int4(uidx, i0, j0, 0));
             }
             if (!h.z.empty()) b->z_given.insert(b->z_given.end(), h.z.begin(), h.z.end());
             if (h.rhs_given) {
