@@ -668,95 +668,330 @@ __global__ void __launch_bounds__(256) k_panel(const UnitDesc *__restrict__ unit
     }
 }
 
-// The same panel factorisation with the panel (rows c0..s-1, NB columns)
-// held in shared memory for the whole kernel: identical operations on
-// identical values, without an L2 round trip in the sequential column loop.
-// Used when (s - c0) * NB * 16 bytes fits in PANEL_SMEM_MAX.
-constexpr int PANEL_SMEM_MAX = 200 * 1024;
-
-__global__ void __launch_bounds__(256) k_panel_smem(const UnitDesc *__restrict__ units, int c0, cx *abuf,
-                                                    int32_t *piv_buf, int32_t *status, int skip_m, const int32_t *__restrict__ order, int base) {
-    // rows padded to PS = NB + 1 entries (distinct banks down a column); the
-    // elimination runs a warp per row and a lane per panel column.  Each
-    // element still receives f = a_rc / a_cc and a_rk -= f a_ck in column
-    // order, as in k_panel.
-    constexpr int PS = NB + 1;
-    extern __shared__ cx s_pan[];  // [m][PS], m = s - c0
-    __shared__ double s_v[8];
-    __shared__ int s_i[8];
-    __shared__ int s_p;
-    int ui = order[base + blockIdx.x];
-    UnitDesc u = units[ui];
-    int s = u.s;
-    if (c0 >= s || s - c0 > skip_m || status[ui] != 0) return;  // skip_m: taller panels go grid-wide
-    int w1 = s + 1;
-    cx *A = abuf + u.a_off;
-    int32_t *piv = piv_buf + u.piv_off;
-    int nb = min(NB, s - c0);
-    int m = s - c0;
-    int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int nw = blockDim.x >> 5;
-    for (int e = tid; e < m * nb; e += blockDim.x) {
-        int rr = e / nb, q = e % nb;
-        s_pan[rr * PS + q] = A[(int64_t)(c0 + rr) * w1 + c0 + q];
-    }
-    __syncthreads();
-    for (int c = c0; c < c0 + nb; ++c) {
-        int lc = c - c0;
-        double bv = -1.0;
-        int bi = -1;
-        for (int r = c + tid; r < s; r += blockDim.x) piv_better(bv, bi, cx_norm(s_pan[(r - c0) * PS + lc]), r);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double ov = __shfl_down_sync(0xffffffffu, bv, o);
-            int oi = __shfl_down_sync(0xffffffffu, bi, o);
-            piv_better(bv, bi, ov, oi);
-        }
-        if (lane == 0) {
-            s_v[wid] = bv;
-            s_i[wid] = bi;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double v = s_v[0];
-            int p = s_i[0];
-            for (int q = 1; q < nw; ++q) piv_better(v, p, s_v[q], s_i[q]);
-            if (p < 0 || v < 1e-30) {
-                status[ui] = -(c + 1);
-                p = -1;
-            }
-            s_p = p;
-            piv[c] = p;
-        }
-        __syncthreads();
-        int p = s_p;
-        if (p < 0) return;
-        if (p != c && tid < nb) {
-            cx t0 = s_pan[lc * PS + tid];
-            s_pan[lc * PS + tid] = s_pan[(p - c0) * PS + tid];
-            s_pan[(p - c0) * PS + tid] = t0;
-        }
-        __syncthreads();
-        const cx pj = lane < nb ? s_pan[lc * PS + lane] : cx_make(0.0, 0.0);
-        const cx diag = s_pan[lc * PS + lc];
-#pragma unroll 2
-        for (int r = c + 1 + wid; r < s; r += nw) {
-            cx *row = s_pan + (r - c0) * PS;
-            cx x = lane < nb ? row[lane] : cx_make(0.0, 0.0);
-            cx f = lane == lc ? cx_div(x, diag) : x;  // one division, then broadcast
-            f = cx_make(__shfl_sync(0xffffffffu, f.re, lc), __shfl_sync(0xffffffffu, f.im, lc));
-            if (lane == lc) row[lc] = f;
-            else if (lane > lc && lane < nb) row[lane] = cx_sub(x, cx_mul(f, pj));
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < m * nb; e += blockDim.x) {
-        int rr = e / nb, q = e % nb;
-        A[(int64_t)(c0 + rr) * w1 + c0 + q] = s_pan[rr * PS + q];
-    }
+__device__ __forceinline__ void cp_async_cx(cx *dst, const cx *src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// Panels taller than one CTA's shared memory: the grid-wide panel of
+// The panel factorisation of systems up to CP_MAX_CTAS * CP_MAX_ROWS rows: a
+// thread per row, the panel in shared memory, the 16 columns being factored
+// in registers, and a cluster of CTAs where one CTA's rows do not suffice.
+// A column's latency is what bounds it (one system) or the FP64 work of the
+// rows (many), so a column takes two barriers and no square root:
+// - Rows never move.  Each thread carries the position its row has reached
+//   (pos); the pivot's becomes c, and the row that stood at c takes the
+//   pivot's.  Rows are written to their positions at the end.
+// - The pivot is the largest hypot, the last of equals (piv_better).  Rows
+//   are first compared by the high word of re^2 + im^2: a row whose word is
+//   two or more below the largest is smaller by 2^-21, relative, and its
+//   hypot (within an ulp of exact) is smaller too.  With one row left it is
+//   the pivot; otherwise, and where the squares leave the safe range, the
+//   hypots are compared as the reference does.
+// - The quotients f = a / diag share the reciprocal of |diag|^2 (Markstein's
+//   correction, as div_by), correctly rounded inside its exponent range.
+// Every element receives f = a_rc / a_cc and a_rk -= f a_ck in column order,
+// as in k_panel; the second 16 columns take the first 16 columns' updates in
+// the same order before they are factored.
+// Measured, factor phase, against one CTA of 256 threads per panel with a
+// warp per row and the panel, hypots and divisions from shared memory:
+// one N = 255 system 2.04 -> 0.70 ms, 512 random antennas 25.4 -> 10.6 ms,
+// 20 x 20 mesh (S = 2520) 19.0 -> 11.8 ms.  About 2,500 cycles a column;
+// spreading a short panel over more CTAs costs more in cluster barriers than
+// its shorter columns give (N = 255: 0.71 at 256 rows a CTA, 0.84 at 64).
+constexpr int CP_MAX_ROWS = 384;  // rows (threads) per CTA: 512 B of panel each
+constexpr int CP_MAX_CTAS = 8;    // the portable cluster size
+constexpr int CP_W = 16;          // columns held in registers
+
+struct alignas(16) CpRow {  // a candidate pivot row and what the choice needs
+    uint32_t hi;            // high word of |a[0]|^2, plus one (0: no row)
+    int cnt;                // 1: no other row within the margin
+    int pos;                // the row's position
+    int pad;
+    double z;               // 1 / |a[0]|^2 (recip_rn)
+    double v;               // slow path: hypot of a[0]
+    cx a[CP_W];             // its entries from the current column on
+};
+constexpr int CP_WARPS = CP_MAX_ROWS / 32;
+struct alignas(16) CpShared {
+    CpRow warp[2][CP_WARPS];    // each warp's candidate, by column parity
+    CpRow cta[2][CP_MAX_CTAS];  // each CTA's, written by the CTAs of the cluster
+    double w_v[CP_WARPS];
+    int w_pos[CP_WARPS];
+    int pos_of[CP_MAX_ROWS];
+};
+static size_t cp_smem(int rows) { return sizeof(CpShared) + sizeof(cx) * NB * (size_t)(rows + 1); }
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16-byte store to the same shared-memory address of CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster(void *p, uint32_t rank, uint4 v) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    uint32_t ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(ra), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
+// 1/x rounded to nearest for 2^-400 <= x < 2^400 whose mantissa is not all
+// ones: a first guess (2^-20), two Newton steps and Markstein's last one,
+// without the branch of a general division, so that it overlaps the column
+// updates beside it.
+__device__ __forceinline__ double recip_rn(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+#pragma unroll
+    for (int q = 0; q < 3; ++q) y = D_FMA(D_FMA(-x, y, 1.0), y, y);
+    return y;
+}
+
+// num-complex's a / b for the quotients of one pivot b: ns = |b|^2 and
+// z = recip_rn(ns).  Each quotient is corrected from z (div_by) where the
+// residuals stay normal, else divided as it stands.
+__device__ __forceinline__ cx cp_div(cx a, cx b, double ns, double z) {
+    const double re = D_ADD(D_MUL(a.re, b.re), D_MUL(a.im, b.im));
+    const double im = D_SUB(D_MUL(a.im, b.re), D_MUL(a.re, b.im));
+    auto ok = [](double v) {  // 2^-400 <= |v| < 2^400
+        const uint32_t k = fnec_libm::lm_hi(v) & 0x7fffffffu;
+        return k - 0x26f00000u < 0x58f00000u - 0x26f00000u;
+    };
+    if (ok(ns) && (uint32_t)fnec_libm::lm_bits(ns) != 0xffffffffu && (ok(re) || re == 0.0) && (ok(im) || im == 0.0))
+        return cx_make(div_by(re, {ns, z}), div_by(im, {ns, z}));
+    return cx_make(D_DIV(re, ns), D_DIV(im, ns));
+}
+
+// The exact choice among a CTA's rows (piv_better over hypots): out of line,
+// the column loop seldom needs it.  The warps' winners go through sh.w_*;
+// `clustered` waits for the whole cluster, whose CTAs have then all read the
+// column's first candidates.
+__device__ __noinline__ int exact_pivot(CpShared &sh, cx a0, int pos, bool act, int nw, bool clustered, double *v_out) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double v = -1.0;
+    int p = -1;
+    if (act) piv_better(v, p, cx_norm(a0), pos);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, p, o);
+        piv_better(v, p, ov, oi);
+    }
+    if (lane == 0) {
+        sh.w_v[wid] = v;
+        sh.w_pos[wid] = p;
+    }
+    if (clustered) cluster_barrier();
+    else __syncthreads();
+    v = -1.0;
+    p = -1;
+    for (int q = 0; q < nw; ++q) piv_better(v, p, sh.w_v[q], sh.w_pos[q]);
+    *v_out = v;
+    return p;
+}
+
+// One system per cluster of nc CTAs (CL: nc > 1).
+template <bool CL>
+__global__ void __launch_bounds__(CP_MAX_ROWS, 1) k_panel_cluster(const UnitDesc *__restrict__ units, int c0, cx *abuf,
+                                                               int32_t *piv_buf, int32_t *status,
+                                                               const int32_t *__restrict__ order, int base, int nc) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    CpShared &sh = *reinterpret_cast<CpShared *>(s_raw);
+    cx *s_f = reinterpret_cast<cx *>(s_raw + sizeof(CpShared));  // [NB][T + 1], by data row
+    const int T = blockDim.x, ld = T + 1, nw = T >> 5;
+    const int rank = CL ? (int)cluster_rank() : 0;
+    const int ui = order[base + blockIdx.x / nc];
+    const UnitDesc u = units[ui];
+    const int s = u.s;
+    if (c0 >= s || status[ui] != 0) return;  // the same in every CTA of the cluster
+    const int w1 = s + 1, nb = min(NB, s - c0), m = s - c0;
+    cx *A = abuf + u.a_off;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int row0 = rank * T, nl = max(0, min(T, m - row0));  // this CTA's rows
+    for (int e = tid; e < nl * nb; e += T) {
+        const int rr = e / nb, q = e % nb;
+        cp_async_cx(&s_f[q * ld + rr], &A[(int64_t)(c0 + row0 + rr) * w1 + c0 + q]);
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    if (CL) cluster_barrier();  // every CTA runs before its shared memory is written
+    else __syncthreads();
+    const bool mine = tid < nl;
+    int pos = c0 + row0 + tid;  // the row's current position
+    int ord = mine ? NB : -1;   // the panel column it became the pivot of; NB: none yet, -1: no row
+    // a row of this CTA to the same place in every CTA of the cluster, by
+    // `n` threads of index `t` (the row is visible to them)
+    auto spread = [&](const CpRow *from, CpRow *to, int t, int n) {
+        constexpr int Q = sizeof(CpRow) / 16;
+        for (int e = t; e < Q * nc; e += n) st_cluster((uint4 *)to + e % Q, e / Q, ((const uint4 *)from)[e % Q]);
+    };
+    int par = 0;
+    for (int h = 0; h * CP_W < nb; ++h) {
+        const int hb = h * CP_W, ncol = min(CP_W, nb - hb);
+        cx a[CP_W];
+#pragma unroll
+        for (int k = 0; k < CP_W; ++k) a[k] = mine && k < ncol ? s_f[(hb + k) * ld + tid] : cx_make(0.0, 0.0);
+        // the earlier half's updates, pivot by pivot
+        for (int c = 0; c < hb; ++c, par ^= 1) {
+            if (ord == c) {
+#pragma unroll
+                for (int k = 0; k < CP_W; ++k) sh.warp[par][0].a[k] = a[k];
+            }
+            const CpRow *src = &sh.warp[par][0];
+            if (CL) {
+                src = &sh.cta[par][0];
+                const bool owner = __any_sync(0xffffffffu, ord == c);
+                __syncwarp();
+                if (owner) spread(&sh.warp[par][0], &sh.cta[par][0], lane, 32);
+                cluster_barrier();
+            } else {
+                __syncthreads();
+            }
+            if (ord > c) {
+                const cx f = s_f[c * ld + tid];
+#pragma unroll
+                for (int k = 0; k < CP_W; ++k) a[k] = cx_sub(a[k], cx_mul(f, src->a[k]));
+            }
+        }
+        if (mine && ord < hb) {
+#pragma unroll
+            for (int k = 0; k < CP_W; ++k)
+                if (k < ncol) s_f[(hb + k) * ld + tid] = a[k];
+        }
+        // |a[0]|^2, its reciprocal, and the warp's candidate among its rows
+        // without a pivot; the reciprocal and the reductions overlap the
+        // updates of the other columns when these follow in the same pass
+        double n2 = 0.0, z = 0.0;
+        unsigned near = 0, top = 0;
+        uint32_t wm = 0;
+        auto choose = [&](bool act) {
+            n2 = D_ADD(D_MUL(a[0].re, a[0].re), D_MUL(a[0].im, a[0].im));
+            z = recip_rn(n2);
+            const uint32_t key = act ? min(fnec_libm::lm_hi(n2) & 0x7fffffffu, 0x7ff00000u) : 0u;
+            wm = __reduce_max_sync(0xffffffffu, key);
+            near = __ballot_sync(0xffffffffu, act && key + 1 >= wm);
+            top = __ballot_sync(0xffffffffu, act && key == wm);
+        };
+        auto announce = [&](int pr) {
+            CpRow &w = sh.warp[pr][wid];
+            if (lane == (top ? __ffs(top) - 1 : 0)) {
+#pragma unroll
+                for (int k = 0; k < CP_W; ++k) w.a[k] = a[k];
+                w.z = z;
+                w.hi = top ? wm + 1 : 0;
+                w.cnt = __popc(near);
+                w.pos = pos;
+            }
+        };
+        choose(ord > hb);
+        announce(par);
+        for (int lc = 0; lc < ncol; ++lc, par ^= 1) {
+            const int col = hb + lc;
+            const bool act = ord > col;
+            __syncthreads();
+            // the largest of n candidates: one is set if no other comes near it
+            uint32_t gm;
+            int best, p;
+            bool one;
+            auto largest = [&](const CpRow *cand, int n) {
+                const uint4 in = lane < n ? *reinterpret_cast<const uint4 *>(cand + lane) : make_uint4(0, 0, 0, 0);
+                gm = __reduce_max_sync(0xffffffffu, in.x);
+                best = __ffs(__ballot_sync(0xffffffffu, in.x == gm)) - 1;
+                const unsigned cn = __ballot_sync(0xffffffffu, in.x + 1 >= gm && (lane == best || in.x > 0));
+                one = __popc(cn) == 1 && __shfl_sync(0xffffffffu, (int)in.y, best) == 1;
+                p = __shfl_sync(0xffffffffu, (int)in.z, best);
+            };
+            largest(sh.warp[par], nw);
+            const CpRow *piv = &sh.warp[par][best];
+            if (CL) {  // the same among the CTAs
+                if (tid == 0 && !one) sh.warp[par][best].cnt = 2;
+                if (wid == 0) {
+                    __syncwarp();
+                    spread(piv, &sh.cta[par][rank], lane, 32);
+                }
+                cluster_barrier();
+                largest(sh.cta[par], nc);
+                piv = &sh.cta[par][best];
+            }
+            // near ties, squares out of range, a column near the singular bound
+            if (!one || gm - 1 >= 0x7ff00000u || gm - 1 < 0x34100000u) {
+                double v;
+                p = exact_pivot(sh, a[0], pos, act, nw, CL, &v);
+                if (p < 0 ? tid == 0 : act && pos == p) {  // the CTA's candidate, in warp slot 0
+                    CpRow &w = sh.warp[par][0];
+#pragma unroll
+                    for (int k = 0; k < CP_W; ++k) w.a[k] = a[k];
+                    w.z = z;
+                    w.v = v;
+                    w.pos = p;
+                }
+                __syncthreads();
+                piv = &sh.warp[par][0];
+                if (CL) {
+                    if (wid == 0) spread(piv, &sh.cta[par][rank], lane, 32);
+                    cluster_barrier();
+                    v = -1.0;
+                    p = -1;
+                    best = 0;
+                    for (int q = 0; q < nc; ++q) {
+                        const int before = p;
+                        piv_better(v, p, sh.cta[par][q].v, sh.cta[par][q].pos);
+                        if (p != before) best = q;
+                    }
+                    piv = &sh.cta[par][best];
+                }
+                // linear.rs:1354 singular test on the chosen pivot (NaN never passes <)
+                if (p < 0 || v < 1e-30) p = -1;
+            }
+            if (rank == 0 && tid == 0) {
+                piv_buf[u.piv_off + c0 + col] = p;
+                if (p < 0) status[ui] = -(c0 + col + 1);
+            }
+            if (p < 0) return;  // the same in every CTA of the cluster
+            const cx *prow = piv->a;
+            const int left = ncol - lc;  // columns left, this one included
+            cx f = cx_make(0.0, 0.0);
+            const bool row = act && pos != p;  // a row below the pivot
+            if (act && !row) {                 // the pivot row: its entries are final
+                ord = col;
+                pos = c0 + col;
+#pragma unroll
+                for (int k = 0; k < CP_W; ++k)
+                    if (k < left) s_f[(col + k) * ld + tid] = a[k];
+            } else if (row) {
+                if (pos == c0 + col) pos = p;
+                const cx diag = prow[0];
+                const double ns = D_ADD(D_MUL(diag.re, diag.re), D_MUL(diag.im, diag.im));
+                f = cp_div(a[0], diag, ns, piv->z);
+                s_f[col * ld + tid] = f;
+                // the columns shift down by one as they are updated
+                a[0] = cx_sub(a[1], cx_mul(f, prow[1]));
+            }
+            if (left > 1) choose(row);
+            if (row) {
+#pragma unroll
+                for (int k0 = 2; k0 < CP_W; k0 += 2) {
+                    if (k0 < left) {
+#pragma unroll
+                        for (int k = k0; k < k0 + 2; ++k) a[k - 1] = cx_sub(a[k], cx_mul(f, prow[k]));
+                    }
+                }
+            }
+            if (left > 1) announce(par ^ 1);
+        }
+    }
+    if (mine) sh.pos_of[tid] = pos;
+    __syncthreads();
+    for (int e = tid; e < nl * nb; e += T) {
+        const int rr = e / nb, q = e % nb;
+        A[(int64_t)sh.pos_of[rr] * w1 + c0 + q] = s_f[q * ld + rr];
+    }
+    if (CL) cluster_barrier();
+}
+
+// Panels taller than the largest cluster holds: the grid-wide panel of
 // fnec_grid.cuh over gridDim.x CTAs per unit (gridDim.y units, the tallest
 // first), launched cooperatively.  Bit-identical to k_panel.
 struct ExactPanelOps {
@@ -945,11 +1180,6 @@ struct PieceCursor {  // columns j0 .. j0 + BP - 1 of row i
         }
     }
 };
-
-__device__ __forceinline__ void cp_async_cx(cx *dst, const cx *src) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
 
 // All BS_THREADS threads; ring: BP_RING * BP_SLOT entries of shared memory.
 __device__ __forceinline__ void backsub_rows(const cx *A, int s, int w1, const cx *bv, int64_t b_stride,
@@ -1599,21 +1829,43 @@ void step_classes(const GridPlan &gp, int c0, int i_begin, std::vector<StepClass
     }
 }
 
+// One cluster per unit, rows dealt evenly over its CTAs.
+static void launch_panel_cluster(const UnitDesc *units, int n, int m_max, int c0, cx *A, int32_t *piv, int32_t *status,
+                                 const int32_t *order, int base, cudaStream_t st) {
+    int nc = 1;
+    while (nc * CP_MAX_ROWS < m_max) nc *= 2;
+    const int rows = ((m_max + nc - 1) / nc + 31) / 32 * 32;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n * nc);
+    cfg.blockDim = dim3(rows);
+    cfg.dynamicSmemBytes = cp_smem(rows);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = nc;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = nc > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, nc > 1 ? k_panel_cluster<true> : k_panel_cluster<false>, units, c0, A, piv, status, order,
+                       base, nc);
+}
+
 uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const GridPlan &gp, cx *A,
                              int32_t *piv, int32_t *status, cudaStream_t st) {
     uint64_t L = 0;
     set_smem_limit_once(k_trailing, (int)TRAILING_SMEM);  // once per device
-    set_smem_limit_once(k_panel_smem, PANEL_SMEM_MAX);
+    set_smem_limit_once(k_panel_cluster<false>, (int)cp_smem(CP_MAX_ROWS));
+    set_smem_limit_once(k_panel_cluster<true>, (int)cp_smem(CP_MAX_ROWS));
     set_smem_limit_once(k_panel_grid, 96 * 1024);
     (void)nu;
-    const int thr_rows = PANEL_SMEM_MAX / (int)((NB + 1) * sizeof(cx));
+    const int thr_rows = CP_MAX_ROWS * CP_MAX_CTAS;
     const int32_t *ord = gp.d_order;
     if (gp.d_sync) cudaMemsetAsync(gp.d_sync, 0, grid_sync_bytes(gp.steps), st);
     std::vector<StepClass> cls;
     for (int c0 = 0; c0 < max_s; c0 += NB) {
         // panels: the tallest units (m > thr_rows) grid-wide or one CTA each
-        // from global memory, the rest one CTA each from shared memory, in
-        // size classes so that short panels do not reserve tall panels' memory
+        // from global memory, the rest a cluster each, in size classes so
+        // that short panels do not reserve tall panels' memory
         int n_thr = 0;
         while (n_thr < (int)gp.s_desc.size() && gp.s_desc[n_thr] - c0 > thr_rows) ++n_thr;
         if (n_thr > 0) {
@@ -1634,8 +1886,7 @@ uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const Gri
         }
         step_classes(gp, c0, n_thr, cls);
         for (const StepClass &c : cls) {
-            k_panel_smem<<<c.i1 - c.i0, 256, sizeof(cx) * (size_t)c.m_max * (NB + 1), st>>>(units, c0, A, piv, status,
-                                                                                      INT_MAX, ord, c.i0);
+            launch_panel_cluster(units, c.i1 - c.i0, c.m_max, c0, A, piv, status, ord, c.i0, st);
             ++L;
         }
         // deferred swaps + U12, then the trailing update, by size class
