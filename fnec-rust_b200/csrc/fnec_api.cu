@@ -3164,7 +3164,7 @@ int64_t request_bytes(const HostAnt &h, int precision) {
     }
     if (s > 380) b += (int64_t)grid_xchg_bytes() + (int64_t)grid_sync_bytes((int)((s + 31) / 32));  // grid panels
     if (precision == FNEC_PRECISION_MIXED && s >= 1536)   // grid-wide GMRES scratch
-        b += 16 * n * ((n + 255) / 256) + 64 * s + 16 * 2 * 296 * 25 + 4096;
+        b += 16 * n * ((n + 255) / 256) + 96 * s + 16 * 2 * 256 * (s + 256) + 16 * 2 * 296 * 25 + 8192;
     return b + (1 << 20);
 }
 

@@ -1938,11 +1938,14 @@ __device__ __forceinline__ cx ldcg_cx(const cx *p) {
     return {d.x, d.y};
 }
 
+constexpr int GI = 256;  // rows of the diagonal blocks the grid-wide substitution inverts
+
 struct GGrid {
     GmresCtx g;
     const int32_t *ccptr, *ccq, *perm;
+    const cx *inv = nullptr;  // inverses of the factor's GI-row diagonal blocks; null: substitution in 32-row blocks
     cx *part;
-    cx *y;
+    cx *y, *y2;     // substitution vectors (y2 with inv only)
     cx *red;
     GridSync *gs;
     int32_t *status;
@@ -2048,9 +2051,75 @@ __device__ bool gg_apply(GGrid &c, const cx *v, cx *out) {
     return true;
 }
 
+// y[r] -= sum_q lu[r][c0 + q] x[q] for rows r0 <= r < r1, x the nb solved
+// entries in shared memory: a warp per row, a row's segment 8 loads a lane.
+__device__ __forceinline__ void gg_update(GGrid &c, cx *y, const cx *sx, int r0, int r1, int c0, int nb) {
+    const GmresCtx &g = c.g;
+    for (int r = r0 + c.gw; r < r1; r += c.TW) {
+        const float2 *row = g.lu + (int64_t)r * g.s + c0;
+        float2 l[GI / 32];
+#pragma unroll
+        for (int q = 0; q < GI / 32; ++q) l[q] = c.lane + 32 * q < nb ? row[c.lane + 32 * q] : cf(0.f, 0.f);
+        const cx yr = ldcg_cx(y + r);
+        cx acc = {0, 0};
+#pragma unroll
+        for (int q = 0; q < GI / 32; ++q) acc = zadd(acc, zmul(f2z(l[q]), sx[c.lane + 32 * q]));
+        acc = warp_sum(acc);
+        if (c.lane == 0) y[r] = zsub(yr, acc);
+    }
+}
+
+// x = inv y for one diagonal block (lower: columns up to the row, else from it)
+__device__ __forceinline__ void gg_block_solve(GGrid &c, const cx *inv, const cx *y, cx *x, int nb, bool lower) {
+    for (int i = c.gw; i < nb; i += c.TW) {
+        const cx *row = inv + (int64_t)i * GI;
+        cx acc = {0, 0};
+        const int b = lower ? 0 : (i & ~31), e = lower ? i + 1 : nb;
+        for (int q = b + c.lane; q < e; q += 32)
+            if (q >= (lower ? 0 : i)) acc = zadd(acc, zmul(row[q], ldcg_cx(y + q)));
+        acc = warp_sum(acc);
+        if (c.lane == 0) x[i] = acc;
+    }
+}
+
+// out = (L U)^-1 P in through the diagonal blocks' inverses: a block's
+// entries are one matrix-vector product over the whole grid, the rows
+// outside it another, so a substitution takes two grid barriers per GI rows
+// and streams the factor once.  Before, one warp solved each 32-row block
+// by a shuffle chain while the grid waited, and that chain and its barrier
+// bounded the whole refinement.  The inverses are FP64, so this is the same
+// operator to FP64 rounding (results agree to 2e-14).  GI: at 256 a block's
+// inverse adds 4 KB a row to the 2 x 8 S bytes of the factor's.
+// Measured, refinement phase: 46 x 46 mesh (S = 12,972) 67.9 -> 21.0 ms,
+// 20 x 20 (S = 2520) 8.15 -> 2.28 ms, 16 x 16 (S = 1632) 5.0 -> 1.5 ms.
+__device__ bool gg_prec_inv(GGrid &c, const cx *in, cx *out) {
+    const int s = c.g.s, nblk = (s + GI - 1) / GI;
+    __shared__ cx s_x[GI];
+    for (int i = c.gt; i < s; i += c.T) c.y[i] = ldcg_cx(in + c.perm[i]);
+    GG_SYNC(c);
+    for (int dir = 0; dir < 2; ++dir) {  // forward y -> y2, then backward y2 -> y
+        cx *y = dir ? c.y2 : c.y, *x = dir ? c.y : c.y2;
+        for (int t = 0; t < nblk; ++t) {
+            const int bk = dir ? nblk - 1 - t : t, c0 = bk * GI, nb = min(GI, s - c0);
+            gg_block_solve(c, c.inv + ((int64_t)bk * 2 + dir) * GI * GI, y + c0, x + c0, nb, dir == 0);
+            GG_SYNC(c);
+            if (t + 1 == nblk) break;
+            for (int i = c.tid; i < GI; i += blockDim.x) s_x[i] = i < nb ? ldcg_cx(x + c0 + i) : cx{0, 0};
+            __syncthreads();
+            if (dir == 0) gg_update(c, y, s_x, c0 + nb, s, c0, nb);
+            else gg_update(c, y, s_x, 0, c0, c0, nb);
+            GG_SYNC(c);
+        }
+    }
+    for (int i = c.gt; i < s; i += c.T) out[i] = ldcg_cx(c.y + i);
+    GG_SYNC(c);
+    return true;
+}
+
 // out = (L U)^-1 P in (the caller has synchronised after writing in);
 // FP64 substitution with the FP32 factor, as apply_prec.
 __device__ bool gg_prec(GGrid &c, const cx *in, cx *out) {
+    if (c.inv) return gg_prec_inv(c, in, out);
     const GmresCtx &g = c.g;
     const int s = g.s, nblk = (s + 31) / 32;
     __shared__ cx s_yb[32];
@@ -2334,8 +2403,8 @@ __global__ void __launch_bounds__(256) k_gmres_grid(const UnitDesc *__restrict__
                                                     const cx *__restrict__ rhs, const double *__restrict__ cosv,
                                                     const float2 *__restrict__ a32buf, const int32_t *__restrict__ pivbuf,
                                                     cx *xbuf, cx *vbuf, cx *wbuf, int32_t *status,
-                                                    const int32_t *__restrict__ perm, cx *part, cx *ybuf, cx *red,
-                                                    GridSync *gs) {
+                                                    const int32_t *__restrict__ perm, const cx *__restrict__ inv,
+                                                    cx *part, cx *ybuf, cx *y2buf, cx *red, GridSync *gs) {
     UnitDesc u = units[ui];
     if (status[u.sys] != 0) return;
     AntDesc a = ants[u.ant];
@@ -2360,8 +2429,10 @@ __global__ void __launch_bounds__(256) k_gmres_grid(const UnitDesc *__restrict__
     c.ccptr = ibuf + a.ccptr_off;
     c.ccq = ibuf + a.ccq_off;
     c.perm = perm;
+    c.inv = inv;
     c.part = part;
     c.y = ybuf;
+    c.y2 = y2buf;
     c.red = red;
     c.gs = gs;
     c.status = &status[u.sys];
@@ -2476,15 +2547,117 @@ __global__ void __launch_bounds__(256, 2) k_gmres_cluster(
 
 // The row permutation of the factor: perm[i] = source row of row i after
 // the swaps piv[0..s) (applied in order, in shared memory when it fits).
+// ---------------------------------------------------------------------------
+// Inverses, in FP64, of the FP32 factor's GI-row diagonal blocks of one
+// system, for the grid-wide refinement: inv[(block * 2 + which) * GI * GI],
+// row-major, which 0 the unit-lower L and 1 the upper U (only the triangle
+// is written).  32-row blocks by substitution, then twice as tall ones from
+// pairs: [L11; L21 L22]^-1 has -L22^-1 L21 L11^-1 below the diagonal, and U
+// correspondingly.  1.1 ms for S = 12,972 in four launches.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(64) k_gi_base(const UnitDesc *__restrict__ units, const MixedUnit *__restrict__ mus,
+                                                int ui, const float2 *__restrict__ a32buf,
+                                                const int32_t *__restrict__ status, cx *inv) {
+    const UnitDesc u = units[ui];
+    if (status[u.sys] != 0) return;
+    __shared__ float2 s_a[32][33];
+    __shared__ cx s_x[2][32][33];
+    const int s = u.s, c0 = blockIdx.x * 32, nb = min(32, s - c0);
+    const float2 *lu = a32buf + mus[ui].a32_off;
+    for (int e = threadIdx.x; e < nb * nb; e += 64) s_a[e / nb][e % nb] = lu[(int64_t)(c0 + e / nb) * s + c0 + e % nb];
+    __syncthreads();
+    const int j = threadIdx.x & 31, which = threadIdx.x >> 5;
+    if (j >= nb) return;
+    cx(*x)[33] = s_x[which];  // lane j reads and writes column j alone
+    cx *o = inv + ((int64_t)(c0 / GI) * 2 + which) * GI * GI + (int64_t)(c0 % GI) * (GI + 1);
+    if (which == 0) {
+        x[j][j] = {1, 0};
+        for (int i = j + 1; i < nb; ++i) {
+            cx acc = {0, 0};
+            for (int k = j; k < i; ++k) acc = zsub(acc, zmul(f2z(s_a[i][k]), x[k][j]));
+            x[i][j] = acc;
+        }
+        for (int i = j; i < nb; ++i) o[(int64_t)i * GI + j] = x[i][j];
+    } else {
+        x[j][j] = zdiv(cx{1, 0}, f2z(s_a[j][j]));
+        for (int i = j - 1; i >= 0; --i) {
+            cx acc = {0, 0};
+            for (int k = i + 1; k <= j; ++k) acc = zsub(acc, zmul(f2z(s_a[i][k]), x[k][j]));
+            x[i][j] = zdiv(acc, f2z(s_a[i][i]));
+        }
+        for (int i = 0; i <= j; ++i) o[(int64_t)i * GI + j] = x[i][j];
+    }
+}
+
+// One 32-column strip of the off-diagonal block of a pair of b-row blocks:
+// grid.x pairs, grid.y strips, grid.z L / U; dynamic shared memory b x 32.
+__global__ void __launch_bounds__(256) k_gi_double(const UnitDesc *__restrict__ units,
+                                                   const MixedUnit *__restrict__ mus, int ui,
+                                                   const float2 *__restrict__ a32buf,
+                                                   const int32_t *__restrict__ status, int b, cx *inv) {
+    extern __shared__ cx s_t[];  // [rows of the strip][32]
+    const UnitDesc u = units[ui];
+    if (status[u.sys] != 0) return;
+    const int s = u.s, c0 = blockIdx.x * 2 * b, which = blockIdx.z;
+    const int n2 = min(b, s - c0 - b);  // rows of the second block
+    const int col = blockIdx.y * 32 + (threadIdx.x & 31), tr = threadIdx.x >> 5;
+    if (n2 <= 0) return;
+    const int rows = which ? b : n2, cols = which ? n2 : b;  // shape of the off-diagonal block
+    if ((int)blockIdx.y * 32 >= cols) return;
+    const float2 *a = a32buf + mus[ui].a32_off + (which ? (int64_t)c0 * s + c0 + b : (int64_t)(c0 + b) * s + c0);
+    cx *blk = inv + ((int64_t)(c0 / GI) * 2 + which) * GI * GI + (int64_t)(c0 % GI) * (GI + 1);
+    const cx *i1 = blk, *i2 = blk + (int64_t)b * (GI + 1);
+    const cx *right = which ? i2 : i1, *left = which ? i1 : i2;
+    cx *out = which ? blk + b : blk + (int64_t)b * GI;
+    const bool live = col < cols;
+    constexpr int R = GI / 2 / 8;  // rows per thread of the tallest strip
+    cx acc[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) acc[q] = {0, 0};
+    // T = off-diagonal block x right inverse (its column's triangle)
+    const int k0 = which ? 0 : (int)blockIdx.y * 32, k1 = which ? min(cols, (int)blockIdx.y * 32 + 32) : cols;
+    for (int k = k0; k < k1; ++k) {
+        const bool in = live && (which ? k <= col : k >= col);
+        const cx v = in ? right[(int64_t)k * GI + col] : cx{0, 0};
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            if (tr + 8 * q < rows) acc[q] = zadd(acc[q], zmul(f2z(a[(int64_t)(tr + 8 * q) * s + k]), v));
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+        if (tr + 8 * q < rows) s_t[(tr + 8 * q) * 32 + (threadIdx.x & 31)] = acc[q];
+    __syncthreads();
+    // out = -left inverse x T
+#pragma unroll
+    for (int q = 0; q < R; ++q) acc[q] = {0, 0};
+    for (int k = 0; k < rows; ++k) {
+        const cx v = s_t[k * 32 + (threadIdx.x & 31)];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const int i = tr + 8 * q;
+            if (i < rows && (which ? k >= i : k <= i)) acc[q] = zsub(acc[q], zmul(left[(int64_t)i * GI + k], v));
+        }
+    }
+    if (live) {
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            if (tr + 8 * q < rows) out[(int64_t)(tr + 8 * q) * GI + col] = acc[q];
+    }
+}
+
 __global__ void k_perm_from_piv(const UnitDesc *__restrict__ units, int ui, const int32_t *__restrict__ pivbuf,
                                 int32_t *perm, int staged) {
     extern __shared__ int32_t s_perm_dyn[];
     UnitDesc u = units[ui];
     const int32_t *piv = pivbuf + u.piv_off;
     int32_t *s_perm = staged ? s_perm_dyn : perm;
-    for (int i = threadIdx.x; i < u.s; i += blockDim.x) s_perm[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0)
+    int moved = 0;  // no row exchange (the Hermitian factor): the identity stands
+    for (int i = threadIdx.x; i < u.s; i += blockDim.x) {
+        s_perm[i] = i;
+        moved |= piv[i] != i;
+    }
+    moved = __syncthreads_or(moved);
+    if (threadIdx.x == 0 && moved)
         for (int c = 0; c < u.s; ++c) {
             int p = piv[c];
             if (p >= 0 && p != c) {
@@ -2625,9 +2798,10 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             partmax = std::max<int64_t>(partmax, (int64_t)((u.n + GG_RC - 1) / GG_RC) * u.n);
         }
         size_t b_perm = sizeof(int32_t) * (size_t)smax, b_part = sizeof(cx) * (size_t)partmax,
-               b_y = sizeof(cx) * (size_t)smax, b_red = sizeof(cx) * 2 * GG_MAX_CTAS * (GM + 1),
+               b_y = sizeof(cx) * (size_t)smax, b_inv = sizeof(cx) * 2 * GI * GI * (size_t)((smax + GI - 1) / GI),
+               b_red = sizeof(cx) * 2 * GG_MAX_CTAS * (GM + 1),
                b_sync = sizeof(GridSync) * w.grid_solves.size();
-        size_t gt = al(b_perm) + al(b_part) + al(b_y) + al(b_red) + al(b_sync);
+        size_t gt = al(b_perm) + al(b_part) + 2 * al(b_y) + al(b_inv) + al(b_red) + al(b_sync);
         e = dev.alloc(&w.grid_base, gt);
         if (e != cudaSuccess) return e;
         unsigned char *q = (unsigned char *)w.grid_base;
@@ -2637,6 +2811,10 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
         q += al(b_part);
         w.g_y = (cx *)q;
         q += al(b_y);
+        w.g_y2 = (cx *)q;
+        q += al(b_y);
+        w.g_inv = (cx *)q;
+        q += al(b_inv);
         w.g_red = (cx *)q;
         q += al(b_red);
         w.g_sync = q;
@@ -2872,10 +3050,21 @@ uint64_t refine_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const Unit
             float2 *a32 = mw.a32;
             cx *vb = mw.v, *wb = mw.w;
             const int32_t *perm = mw.g_perm;
+            const cx *inv = mw.g_inv;
+            {
+                const int sk = mw.grid_s[k];
+                set_smem_limit_once(k_gi_double, (int)(sizeof(cx) * GI / 2 * 32));
+                k_gi_base<<<(sk + 31) / 32, 64, 0, st>>>(d_solves, mw.mu, ui, mw.a32, status, mw.g_inv);
+                for (int b = 32; b < GI; b *= 2)
+                    k_gi_double<<<dim3((sk + 2 * b - 1) / (2 * b), b / 32, 2), 256, sizeof(cx) * b * 32, st>>>(
+                        d_solves, mw.mu, ui, mw.a32, status, b, mw.g_inv);
+                L += 4;
+            }
             void *args[] = {(void *)&d_solves, (void *)&d_ants, (void *)&mus, (void *)&ui, (void *)&ibuf,
                             (void *)&crows, (void *)&z, (void *)&rhs, (void *)&cosv, (void *)&a32,
                             (void *)&piv, (void *)&x, (void *)&vb, (void *)&wb, (void *)&status,
-                            (void *)&perm, (void *)&mw.g_part, (void *)&mw.g_y, (void *)&mw.g_red, (void *)&gs};
+                            (void *)&perm, (void *)&inv, (void *)&mw.g_part, (void *)&mw.g_y, (void *)&mw.g_y2,
+                            (void *)&mw.g_red, (void *)&gs};
             if (mw.grid_ctas <= 0 ||
                 launch_cooperative((const void *)k_gmres_grid, dim3(mw.grid_ctas), dim3(256), args, 0, st) !=
                     cudaSuccess) {

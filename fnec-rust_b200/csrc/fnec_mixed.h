@@ -53,7 +53,8 @@ struct MixedWork {
     void *grid_base = nullptr;     // scratch shared by those launches
     int32_t *g_perm = nullptr;
     cx *g_part = nullptr;
-    cx *g_y = nullptr;
+    cx *g_y = nullptr, *g_y2 = nullptr;  // substitution vectors
+    cx *g_inv = nullptr;                 // inverses of the factor's 256-row diagonal blocks
     cx *g_red = nullptr;
     void *g_sync = nullptr;
     int grid_ctas = 0;

@@ -1,0 +1,33 @@
+"""The grid-wide refinement at the edges of its 256-row diagonal blocks:
+meshes whose S is just above a multiple of 256 or below one, against the
+plain FP64 form (Zin 1e-6, currents 1e-7 normwise: the mixed form's gates)."""
+import numpy as np
+import pytest
+
+import bench
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def acc():
+    import nec_accel
+
+    return nec_accel
+
+
+# a grid of nx x ny cells has 3 (nx (ny + 1) + ny (nx + 1)) unknowns
+@pytest.mark.parametrize("edges,pivoting", [(512, 0), (513, 0), (597, 0), (598, 1), (683, 0), (720, 1)])
+def test_mixed_mesh_matches_plain(acc, edges, pivoting):
+    w, s, f = bench.mesh_workload(19)
+    ant = acc.Antenna(acc.wires_array(w[:edges]), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    plain = acc.HallenBatch([ant]).solve()
+    b = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+    assert b.units[0]["s"] == 3 * edges
+    b.schedule = {"factor_pivoting": pivoting}
+    mixed = b.solve()
+    assert plain.status[0] == 0 and mixed.status[0] == 0
+    x0, x1 = plain.currents[0], mixed.currents[0]
+    assert np.linalg.norm(x1 - x0) <= 1e-7 * np.linalg.norm(x0)
+    z0, z1 = (complex(r.feeds[0][0][5], r.feeds[0][0][6]) for r in (plain, mixed))
+    assert abs(z1 - z0) <= 1e-6 * abs(z0)
