@@ -3158,6 +3158,7 @@ int64_t request_bytes(const HostAnt &h, int precision) {
         if (s - 32 >= 192) {                               // tensor-core trailing stacks and step lists
             const int64_t m0 = s - 32, pa = (m0 + 127) / 128 * 128, pb = (2 * m0 + 127) / 128 * 128;
             b += (256 * (2 * pa + 2 * pb) + 32 * ((s + 31) / 32)) * f;
+            if (s >= 3072) b += (2048 * (pa + pb) + 64 * ((s + 127) / 128) + 1024) * f;  // wide factor steps
         }
     } else {
         b += 16 * s * (s + 1) * f + 4 * s * f;             // FP64 factor, pivots

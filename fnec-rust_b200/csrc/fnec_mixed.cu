@@ -639,6 +639,15 @@ __host__ __device__ constexpr int fu_max_s(int level) { return level <= 0 ? 0 : 
 constexpr int FU_MAX_S_ALL = 512;
 // trailing blocks of at least this many rows go to the tensor cores
 constexpr int TC_TRAIL_MIN_M = 192;
+// Wide steps of the Hermitian factor: at 32 columns a step, reading and
+// writing A22 bounds the trailing update, SIMT or tensor-core (K = 64).
+// Measured, factor phase, 32 against 128 columns: 46 x 46 mesh (S = 12,972)
+// 99.5 -> 43.1 ms (the trailing kernels 87.6 -> 28.6), 30 x 30 (S = 5580)
+// 14.2 -> 10.7, 20 x 20 (2520) 4.24 = 4.24, 16 x 16 (1632) 2.89 < 3.02 ms:
+// hence the bound on S.  The 3xTF32 products leave the refinement's final
+// residual at or below the FP32 tiles' (S = 1632 to 12,972: 0.4 to 0.7 of it).
+constexpr int WIDE = 128;
+constexpr int WIDE_MIN_S = 3072;  // and at most TC_WIDE_MAX_UNITS such units
 constexpr int FU_THREADS = 256;
 constexpr size_t FU_SMEM = sizeof(float2) * (size_t)(MNB * (MNB + 1) + MNB * FU_THREADS);  // the swap stage
 // dynamic shared memory of a launch whose largest unit has S = smax: the
@@ -2906,7 +2915,7 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
         while (n_tc < (int)sd.size() && sd[n_tc] - 32 >= TC_TRAIL_MIN_M) ++n_tc;
         if (n_tc > 0 && w.tc) {
             TcTrailPlan *p = new TcTrailPlan();
-            tc_trail_plan(sd, ord, n_tc, TC_TRAIL_MIN_M, *p);
+            tc_trail_plan(sd, ord, n_tc, TC_TRAIL_MIN_M, 1, *p);
             size_t b_st = sizeof(float) * 32 * (size_t)p->rows, b_u = sizeof(TcTrailUnit) * (p->units.size() + 1);
             size_t tot = 2 * al(b_st) + al(b_u);
             e = dev.alloc(&w.trail_base, tot);
@@ -2928,6 +2937,33 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             }
             w.trail = p;
             w.trail_n = n_tc;
+        }
+        int n_wide = 0;
+        while (n_wide < (int)sd.size() && sd[n_wide] >= WIDE_MIN_S) ++n_wide;
+        if (n_wide > 0 && n_wide <= TC_WIDE_MAX_UNITS && w.tc && tc_wide_ready()) {
+            TcTrailPlan *p = new TcTrailPlan();
+            tc_trail_plan(sd, ord, n_wide, 1, WIDE / MNB, *p);
+            size_t b_st = sizeof(float) * 32 * (size_t)p->rows, b_u = sizeof(TcTrailUnit) * (p->units.size() + 1);
+            size_t tot = 2 * al(b_st) + al(b_u);
+            e = dev.alloc(&w.wide_base, tot);
+            if (e != cudaSuccess) {
+                delete p;
+                return e;
+            }
+            unsigned char *q = (unsigned char *)w.wide_base;
+            w.wd_hi = (float *)q;
+            q += al(b_st);
+            w.wd_lo = (float *)q;
+            q += al(b_st);
+            w.d_wide = q;
+            w.bytes += tot;
+            e = dev.upload(w.d_wide, p->units.data(), sizeof(TcTrailUnit) * p->units.size());
+            if (e != cudaSuccess || !tc_trail_maps(*p, w.wd_hi, w.wd_lo)) {
+                delete p;
+                return e != cudaSuccess ? e : cudaErrorNotSupported;
+            }
+            w.wide = p;
+            w.wide_n = n_wide;
         }
     }
     if (systems.size() >= 4 && !w.fmade) {  // concurrent factor groups
@@ -2959,6 +2995,11 @@ void free_mixed(MixedWork &w, const DevAlloc &dev) {
     dev.release(w.c_base);
     dev.release(w.trail_base);
     w.trail_base = nullptr;
+    dev.release(w.wide_base);
+    w.wide_base = nullptr;
+    delete w.wide;
+    w.wide = nullptr;
+    w.wide_n = 0;
     delete w.trail;
     w.trail = nullptr;
     w.trail_n = 0;
@@ -3147,9 +3188,12 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
     if (gp.unit_factor > 0)
         while (i_unit > 0 && gp.s_desc[i_unit - 1] <= fu_max_s(gp.unit_factor)) --i_unit;
     const bool unit_launch = i_unit < nu_all;
+    // the tallest units of the Hermitian factor take wide steps, ahead of
+    // the others (tensor_trailing 1 and 2 keep 32-column steps for all)
+    const int n_wide = herm && mw.wide && !mw.use_tc_trail && !mw.two_step ? std::min(mw.wide_n, i_unit) : 0;
     int G = std::max(1, std::min(gp.factor_streams, MixedWork::MAX_FACTOR_STREAMS) - (unit_launch ? 1 : 0));
-    if (!mw.fmade || i_unit < 2 * G) G = 1;
-    std::vector<int> gb(1, 0);
+    if (!mw.fmade || i_unit - n_wide < 2 * G) G = 1;
+    std::vector<int> gb(1, n_wide);
     if (G > 1) {
         // units whose panels outgrow one CTA (grid-wide or global-memory
         // panels, one exchange area) all stay in the first group
@@ -3157,8 +3201,8 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
         while (!herm && n_tall < i_unit && gp.s_desc[n_tall] > thr_rows) ++n_tall;
         if (mw.trail && mw.use_tc_trail) n_tall = std::max(n_tall, std::min(mw.trail_n, i_unit));  // one stack set
         double tot = 0, acc = 0;
-        for (int i = 0; i < i_unit; ++i) tot += (double)gp.s_desc[i] * gp.s_desc[i] * gp.s_desc[i];
-        for (int i = 0; i < i_unit && (int)gb.size() < G; ++i) {
+        for (int i = n_wide; i < i_unit; ++i) tot += (double)gp.s_desc[i] * gp.s_desc[i] * gp.s_desc[i];
+        for (int i = n_wide; i < i_unit && (int)gb.size() < G; ++i) {
             acc += (double)gp.s_desc[i] * gp.s_desc[i] * gp.s_desc[i];
             if (acc >= tot * (double)gb.size() / G && i + 1 < i_unit && i + 1 >= n_tall) gb.push_back(i + 1);
         }
@@ -3188,14 +3232,8 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
     }
     std::vector<StepClass> cls;
     const bool two_step = mw.two_step && !(mw.trail && mw.use_tc_trail);
-    for (int grp = 0; grp < G && i_unit > 0; ++grp) {
-    const int gi0 = gb[grp], gi1 = gb[grp + 1];
-    cudaStream_t fs = grp == 0 ? st : mw.fstream[grp - 1];
-    for (int c0 = 0; herm && gi0 < gi1 && c0 < gp.s_desc[gi0]; c0 += MNB) {
-        // Hermitian factor: panel (diagonal block, L21, mirrored U12), then
-        // the trailing tiles on and below the diagonal, per size class: the
-        // largest units' on the tensor cores when tensor_trailing is on (a
-        // prefix of the order, in the first group), the rest as SIMT tiles
+    // the panel step at c0 of units [i0, i1) of the Hermitian factor
+    auto herm_panels = [&](int c0, int gi0, int gi1, cudaStream_t fs) {
         step_classes(gp, c0, gi0, cls, gi1);
         for (const StepClass &c : cls) {
             const int rows = c.m_max - MNB;
@@ -3212,6 +3250,38 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
                 ++L;
             }
         }
+    };
+    // Wide steps: four 32-column panels, each updating only the rest of the
+    // 128 columns, then one tensor-core update of the trailing block with
+    // K = 256, so A22 is read and written once per 128 columns.
+    for (int C0 = 0; n_wide > 0 && C0 < gp.s_desc[0]; C0 += WIDE) {
+        for (int c0 = C0; c0 < std::min(C0 + WIDE, gp.s_desc[0]); c0 += MNB) {
+            herm_panels(c0, 0, n_wide, st);
+            if (c0 + MNB >= C0 + WIDE) continue;
+            step_classes(gp, c0, 0, cls, n_wide);
+            for (const StepClass &c : cls) {
+                const int rows = c.m_max - MNB, cols = C0 + WIDE - c0 - MNB;
+                if (rows <= 0) continue;
+                dim3 g2(((rows + 63) / 64) * ((cols + 63) / 64), c.i1 - c.i0);
+                k_trailing32<<<g2, 256, 0, st>>>(d_units, mw.smu, c0, mw.a32, status, ord, c.i0, 1, C0 + WIDE, 0);
+                ++L;
+            }
+        }
+        if (mw.wide->active(C0 / WIDE) > 0) {
+            tc_trail_run(*mw.wide, C0 / WIDE, n_wide, static_cast<const TcTrailUnit *>(mw.d_wide), d_units, mw.smu,
+                         mw.a32, mw.wd_hi, mw.wd_lo, status, st, true);
+            L += 3;
+        }
+    }
+    for (int grp = 0; grp < G && i_unit > 0; ++grp) {
+    const int gi0 = gb[grp], gi1 = gb[grp + 1];
+    cudaStream_t fs = grp == 0 ? st : mw.fstream[grp - 1];
+    for (int c0 = 0; herm && gi0 < gi1 && c0 < gp.s_desc[gi0]; c0 += MNB) {
+        // Hermitian factor: panel (diagonal block, L21, mirrored U12), then
+        // the trailing tiles on and below the diagonal, per size class: the
+        // largest units' on the tensor cores when tensor_trailing is on (a
+        // prefix of the order, in the first group), the rest as SIMT tiles
+        herm_panels(c0, gi0, gi1, fs);
         const int k_tc =
             (grp == 0 && mw.trail && mw.use_tc_trail) ? std::min(mw.trail->active(c0 / MNB), i_unit) : 0;
         step_classes(gp, c0, std::max(gi0, k_tc), cls, gi1);

@@ -87,6 +87,13 @@ struct MixedWork {
     float *tr_hi = nullptr, *tr_lo = nullptr;
     void *d_trail = nullptr;  // TcTrailUnit per (step, unit)
     int trail_n = 0;          // units (a prefix of the s-descending order) it covers
+    // 128-column steps of the Hermitian factor's tallest units (a prefix of
+    // the order), always on the tensor cores
+    TcTrailPlan *wide = nullptr;
+    void *wide_base = nullptr;
+    float *wd_hi = nullptr, *wd_lo = nullptr;
+    void *d_wide = nullptr;
+    int wide_n = 0;
     bool use_tc_trail = false; // the tuner picks it
     bool two_step = false;     // SIMT trailing updates once per two steps (look-ahead of the next panel)
     bool pivoting = false;     // GEPP with row exchanges; else the Hermitian factor without them

@@ -182,8 +182,8 @@ __device__ __forceinline__ void epi_gram(const TcTile &t, const TcEpilogue &ep, 
     }
 }
 
-// A22 -= D for one factor step: rows c0 + 32 + tile row, float columns
-// 2 (c0 + 32) + tile column of the unit's interleaved complex A32.  The
+// A22 -= D for one factor step: rows r0 + tile row, float columns
+// 2 r0 + tile column of the unit's interleaved complex A32.  The
 // warp's 32 x 32 block (a row per lane from TMEM) is transposed through
 // shared memory (stg: 32 x 33 floats of the warp) so that each
 // read-modify-write covers 32 consecutive floats of one row.
@@ -195,8 +195,8 @@ __device__ __forceinline__ void epi_trail(const TcTile &t, const TcEpilogue &ep,
     __syncwarp();
     const int s = ep.units[t.unit].s;
     float *A = reinterpret_cast<float *>(ep.a32 + ep.mus[t.unit].a32_off);
-    const int64_t F = 2 * ((int64_t)ep.c0 + 32) + (int64_t)t.tj * NT + col + lane;
-    const int64_t R0 = (int64_t)ep.c0 + 32 + (int64_t)t.ti * BM + row0;
+    const int64_t F = 2 * (int64_t)ep.r0 + (int64_t)t.tj * NT + col + lane;
+    const int64_t R0 = (int64_t)ep.r0 + (int64_t)t.ti * BM + row0;
     // all reads (the transposed block, then A22) before any write, so no
     // load waits behind a store it might alias
     float d[32], a[32];
@@ -364,14 +364,19 @@ constexpr size_t pt_smem() {
            (EPI == TC_EPI_TRAIL ? PT_EPI_WARPS * 32 * 33 * sizeof(float) : 0) + 1024;
 }
 
+// units per step: few for the wide steps, whose stages leave 1 KB of shared memory
+template <int EPI, int NT>
+constexpr int pt_max_units = EPI == TC_EPI_TRAIL && NT == BN ? TC_WIDE_MAX_UNITS : PT_MAX_UNITS;
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // Tile g of the step's sequence: its unit entry and grid position (false:
 // g is past the end or, with lower, the tile lies wholly above the diagonal)
+template <int NT>
 __device__ __forceinline__ bool pt_tile(const TcTrailUnit *tl, const int32_t *pre, int na, int g, bool lower,
-                                        TcTile &t) {
+                                        int kblocks, TcTile &t) {
     if (g >= pre[na]) return false;
     int lo = 0, hi = na;  // pre[lo] <= g < pre[hi]
     while (hi - lo > 1) {
@@ -380,13 +385,13 @@ __device__ __forceinline__ bool pt_tile(const TcTrailUnit *tl, const int32_t *pr
         else hi = mid;
     }
     const TcTrailUnit tu = tl[lo];
-    const int ntj = tu.n2_pad / TRAIL_NT, x = g - pre[lo], ti = x / ntj, tj = x % ntj;
-    if (lower && (TRAIL_NT / 2) * tj > BM * ti + BM - 1) return false;
+    const int ntj = tu.n2_pad / NT, x = g - pre[lo], ti = x / ntj, tj = x % ntj;
+    if (lower && (NT / 2) * tj > BM * ti + BM - 1) return false;
     t.a_row = (int32_t)(tu.a_base + (int64_t)ti * BM);
-    t.b_row = (int32_t)(tu.b_base + (int64_t)tj * TRAIL_NT);
+    t.b_row = (int32_t)(tu.b_base + (int64_t)tj * NT);
     t.a_kstride = tu.m_pad;
     t.b_kstride = tu.n2_pad;
-    t.kblocks = 2;
+    t.kblocks = kblocks;
     t.unit = tu.unit;
     t.ti = ti;
     t.tj = tj;
@@ -395,15 +400,15 @@ __device__ __forceinline__ bool pt_tile(const TcTrailUnit *tl, const int32_t *pr
 
 // The next tile of the sequence: the trailing update's tile g (decoded from
 // the step's units), or entry g of the Gram's tile list.
-template <int EPI>
+template <int EPI, int NT>
 __device__ __forceinline__ bool pt_next(const TcTrailUnit *tl, const TcTile *tiles, const int32_t *pre, int na,
-                                        int g, bool lower, TcTile &t) {
-    if (EPI == TC_EPI_TRAIL) return pt_tile(tl, pre, na, g, lower, t);
+                                        int g, bool lower, int kblocks, TcTile &t) {
+    if (EPI == TC_EPI_TRAIL) return pt_tile<NT>(tl, pre, na, g, lower, kblocks, t);
     t = tiles[g];
     return true;
 }
 
-// EPI TC_EPI_TRAIL (NT 64, na units of the step) or TC_EPI_GRAM (NT 128, na
+// EPI TC_EPI_TRAIL (NT 64, or 128 for wider steps; na units of the step) or TC_EPI_GRAM (NT 128, na
 // tiles in `tiles`)
 template <int EPI, int NT>
 __global__ void __launch_bounds__(PT_THREADS, 1)
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1)
     constexpr int PT_STG = 2 * BOX_BYTES + 2 * B_BOX;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_bar[2 * PT_ST + 5];
-    __shared__ int32_t s_pre[PT_MAX_UNITS + 1];
+    __shared__ int32_t s_pre[pt_max_units<EPI, NT> + 1];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_abort_unit;
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -466,7 +471,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1)
         if (lane == 0) {  // TMA producer
             int kq = 0;   // k-blocks issued over the sequence
             for (int g = blockIdx.x; g < total && !*abort_word; g += gridDim.x) {
-                if (!pt_next<EPI>(tl, tiles, s_pre, na, g, lower, t)) continue;
+                if (!pt_next<EPI, NT>(tl, tiles, s_pre, na, g, lower, ep.kblocks, t)) continue;
                 for (int kb = 0; kb < t.kblocks; ++kb, ++kq) {
                     const int st = kq % PT_ST;
                     const uint32_t ph = (uint32_t)(kq / PT_ST) & 1u;
@@ -491,7 +496,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1)
             int kq = 0, i = 0;
             bool ok = true;
             for (int g = blockIdx.x; ok && g < total; g += gridDim.x) {
-                if (!pt_next<EPI>(tl, tiles, s_pre, na, g, lower, t)) continue;
+                if (!pt_next<EPI, NT>(tl, tiles, s_pre, na, g, lower, ep.kblocks, t)) continue;
                 const int b = i & 1;
                 if (i >= 2 && !mbar_wait(tempty(b), (uint32_t)((i >> 1) - 1) & 1u, abort_word, wlim)) {
                     s_abort_unit = t.unit;
@@ -534,7 +539,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1)
         float *stg = stage_out + (warp - 2) * 32 * 33;
         int i = 0;
         for (int g = blockIdx.x; g < total; g += gridDim.x) {
-            if (!pt_next<EPI>(tl, tiles, s_pre, na, g, lower, t)) continue;
+            if (!pt_next<EPI, NT>(tl, tiles, s_pre, na, g, lower, ep.kblocks, t)) continue;
             const int b = i & 1;
             if (!mbar_wait(tfull(b), (uint32_t)(i >> 1) & 1u, abort_word, wlim)) {
                 if (lane == 0) s_abort_unit = t.unit;
@@ -610,8 +615,9 @@ __global__ void k_split_gram(const UnitDesc *__restrict__ units, const TcGramUni
     }
 }
 
-// L21 of one factor step -> the trailing A operand (K-blocked hi/lo):
-// k-block 0 the real parts, k-block 1 the imaginary parts, a warp per row.
+// L21 of one factor step -> the trailing A operand (K-blocked hi/lo): for
+// part p = blockIdx.z (columns c0 + 32 p ..) k-block 2p the real parts,
+// 2p + 1 the imaginary parts, a warp per row; gridDim.z parts.
 __global__ void k_split_trail_a(const TcTrailUnit *__restrict__ tu_list, const UnitDesc *__restrict__ systems,
                                 const MixedUnit *__restrict__ smu, const float2 *__restrict__ a32buf, int c0,
                                 float *hi, float *lo) {
@@ -620,9 +626,11 @@ __global__ void k_split_trail_a(const TcTrailUnit *__restrict__ tu_list, const U
     if (i >= tu.m_pad) return;
     const int s = systems[tu.unit].s;
     float2 v = make_float2(0.f, 0.f);
-    if (i < tu.m) v = a32buf[smu[tu.unit].a32_off + (int64_t)(c0 + 32 + i) * s + c0 + k];
+    const int cp = c0 + 32 * blockIdx.z, r0 = c0 + 32 * gridDim.z;
+    if (i < tu.m) v = a32buf[smu[tu.unit].a32_off + (int64_t)(r0 + i) * s + cp + k];
     float h, l;
-    const int64_t o0 = (tu.a_base + i) * 32 + k, o1 = (tu.a_base + tu.m_pad + i) * 32 + k;
+    const int64_t kb = 2 * blockIdx.z;
+    const int64_t o0 = (tu.a_base + kb * tu.m_pad + i) * 32 + k, o1 = o0 + (int64_t)tu.m_pad * 32;
     split_tf32(v.x, h, l);
     hi[o0] = h;
     lo[o0] = l;
@@ -632,8 +640,8 @@ __global__ void k_split_trail_a(const TcTrailUnit *__restrict__ tu_list, const U
 }
 
 // U12 of one factor step -> the trailing B operand: rows 2j (Re U, -Im U)
-// and 2j+1 (Im U, Re U) over k-blocks 0 / 1.  A 32 (k) x 32 (j) block of
-// U is transposed through shared memory.
+// and 2j+1 (Im U, Re U) over k-blocks 2p / 2p + 1 of part p = blockIdx.z.
+// A 32 (k) x 32 (j) block of U is transposed through shared memory.
 __global__ void k_split_trail_b(const TcTrailUnit *__restrict__ tu_list, const UnitDesc *__restrict__ systems,
                                 const MixedUnit *__restrict__ smu, const float2 *__restrict__ a32buf, int c0,
                                 float *hi, float *lo) {
@@ -643,9 +651,10 @@ __global__ void k_split_trail_b(const TcTrailUnit *__restrict__ tu_list, const U
     if (2 * j0 >= tu.n2_pad) return;
     const int s = systems[tu.unit].s;
     const float2 *A = a32buf + smu[tu.unit].a32_off;
+    const int cp = c0 + 32 * blockIdx.z, r0 = c0 + 32 * gridDim.z;
     for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
         const int k = e / 32, jj = e % 32, j = j0 + jj;
-        s_u[jj][k] = j < tu.m ? A[(int64_t)(c0 + k) * s + c0 + 32 + j] : make_float2(0.f, 0.f);
+        s_u[jj][k] = j < tu.m ? A[(int64_t)(cp + k) * s + r0 + j] : make_float2(0.f, 0.f);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 64 * 32; e += blockDim.x) {  // 64 B rows (2j + sgn) x 32 k
@@ -656,7 +665,8 @@ __global__ void k_split_trail_b(const TcTrailUnit *__restrict__ tu_list, const U
         const float x0 = sg ? u.y : u.x;   // k-block 0
         const float x1 = sg ? u.x : -u.y;  // k-block 1
         float h, l;
-        const int64_t o0 = (tu.b_base + row) * 32 + k, o1 = (tu.b_base + tu.n2_pad + row) * 32 + k;
+        const int64_t kb = 2 * blockIdx.z;
+        const int64_t o0 = (tu.b_base + kb * tu.n2_pad + row) * 32 + k, o1 = o0 + (int64_t)tu.n2_pad * 32;
         split_tf32(x0, h, l);
         hi[o0] = h;
         lo[o0] = l;
@@ -737,7 +747,9 @@ cudaError_t tc_gram_plan(const std::vector<UnitDesc> &systems, TcGramPlan &p) {
 }
 
 cudaError_t tc_trail_plan(const std::vector<int> &s_desc, const std::vector<int32_t> &order, int n, int min_m,
-                          TcTrailPlan &p) {
+                          int parts, TcTrailPlan &p) {
+    const int width = 32 * parts;
+    p.parts = parts;
     p.units.clear();
     p.u_off.assign(1, 0);
     p.max_tiles.clear();
@@ -747,20 +759,20 @@ cudaError_t tc_trail_plan(const std::vector<int> &s_desc, const std::vector<int3
     std::vector<int64_t> a_base(n), b_base(n);
     int64_t rows = 0;
     for (int q = 0; q < n; ++q) {  // stack rows sized for the unit's first step
-        const int64_t m0 = std::max(0, s_desc[q] - 32);
+        const int64_t m0 = std::max(0, s_desc[q] - width);
         a_base[q] = rows;
-        rows += 2 * (int64_t)pad(m0);
+        rows += 2 * parts * (int64_t)pad(m0);
         b_base[q] = rows;
-        rows += 2 * (int64_t)pad(2 * m0);
+        rows += 2 * parts * (int64_t)pad(2 * m0);
     }
     p.rows = rows;
     const int max_s = n > 0 ? s_desc[0] : 0;
-    for (int c0 = 0; c0 < max_s; c0 += 32) {
+    for (int c0 = 0; c0 < max_s; c0 += width) {
         int32_t mt = 0, mm = 0, mn = 0;
-        for (int q = 0; q < n && s_desc[q] - c0 - 32 >= min_m; ++q) {
+        for (int q = 0; q < n && s_desc[q] - c0 - width >= min_m; ++q) {
             TcTrailUnit t;
             t.unit = order[q];
-            t.m = s_desc[q] - c0 - 32;
+            t.m = s_desc[q] - c0 - width;
             t.m_pad = pad(t.m);
             t.n2_pad = pad(2 * (int64_t)t.m);
             t.a_base = a_base[q];
@@ -784,16 +796,22 @@ bool tc_trail_maps(TcTrailPlan &p, const float *hi, const float *lo) {
     return p.ready;
 }
 
+bool tc_wide_ready() {
+    constexpr size_t wsm = pt_smem<TC_EPI_TRAIL, BN>();
+    return set_smem_limit_once((const void *)k_tc_persist<TC_EPI_TRAIL, BN>, (int)wsm) >= (int)wsm;
+}
+
 cudaError_t tc_trail_run(const TcTrailPlan &p, int step, int count, const TcTrailUnit *d_trail, const UnitDesc *d_systems,
                          const MixedUnit *d_smu, float2 *a32, float *hi, float *lo, int32_t *status, cudaStream_t st,
                          bool lower, bool persistent) {
     const int na = std::min(count, p.active(step));
     if (na <= 0) return cudaSuccess;
     const TcTrailUnit *tl = d_trail + p.u_off[step];
-    const int c0 = 32 * step;
-    k_split_trail_a<<<dim3((unsigned)(p.max_mpad[step] / 8), (unsigned)na), 256, 0, st>>>(tl, d_systems, d_smu, a32,
-                                                                                         c0, hi, lo);
-    k_split_trail_b<<<dim3((unsigned)((p.max_n2pad[step] / 2 + 31) / 32), (unsigned)na), 256, 0, st>>>(
+    const int c0 = 32 * p.parts * step;
+    const unsigned parts = (unsigned)p.parts;
+    k_split_trail_a<<<dim3((unsigned)(p.max_mpad[step] / 8), (unsigned)na, parts), 256, 0, st>>>(tl, d_systems, d_smu,
+                                                                                                a32, c0, hi, lo);
+    k_split_trail_b<<<dim3((unsigned)((p.max_n2pad[step] / 2 + 31) / 32), (unsigned)na, parts), 256, 0, st>>>(
         tl, d_systems, d_smu, a32, c0, hi, lo);
     TcEpilogue ep{};
     ep.units = d_systems;
@@ -801,15 +819,23 @@ cudaError_t tc_trail_run(const TcTrailPlan &p, int step, int count, const TcTrai
     ep.a32 = a32;
     ep.status = status;
     ep.status_of_tile = 1;
-    ep.c0 = c0;
+    ep.r0 = c0 + 32 * p.parts;
+    ep.kblocks = 2 * p.parts;
     ep.trail = tl;
     ep.trail_lower = lower ? 1 : 0;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (p.parts > 1) {
+        constexpr size_t wsm = pt_smem<TC_EPI_TRAIL, BN>();
+        if (na > TC_WIDE_MAX_UNITS || !tc_wide_ready()) return cudaErrorInvalidConfiguration;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (int64_t)p.max_tiles[step] * na));
+        k_tc_persist<TC_EPI_TRAIL, BN><<<grid, PT_THREADS, wsm, st>>>(p.m_hi, p.m_lo, p.m_hi, p.m_lo, nullptr, na, ep);
+        return cudaGetLastError();
+    }
     constexpr size_t psm = pt_smem<TC_EPI_TRAIL, TRAIL_NT>();
     if (persistent && na <= PT_MAX_UNITS &&
         set_smem_limit_once((const void *)k_tc_persist<TC_EPI_TRAIL, TRAIL_NT>, (int)psm) >= (int)psm) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int64_t tiles = (int64_t)p.max_tiles[step] * (BN / TRAIL_NT) * na;  // bound on the sequence
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, tiles));
         k_tc_persist<TC_EPI_TRAIL, TRAIL_NT><<<grid, PT_THREADS, psm, st>>>(p.m_hi, p.m_lo, p.m_hi_b, p.m_lo_b,

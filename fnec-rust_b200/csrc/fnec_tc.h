@@ -38,6 +38,9 @@ struct TcTrailUnit {
     int32_t n2_pad;  // 2m rounded up to 128: B rows per k-block
     int64_t a_base, b_base;  // first rows of the unit's A and B in the stacks
 };
+// A wider step of `parts` 32-column panels has K = 64 parts: k-blocks 2p and
+// 2p + 1 hold part p's columns as above, and the trailing block starts
+// 32 parts below c0.
 
 // One 128x128 output tile.  Operand rows of k-block kb start at
 // a_row + kb * a_kstride (A) and b_row + kb * b_kstride (B) of the
@@ -62,10 +65,11 @@ struct TcEpilogue {
     // both: a CTA whose waits ran out marks status[unit] (or status[0])
     int32_t *status;
     int32_t status_of_tile;
-    // TC_EPI_TRAIL: the step and its units (blockIdx.y), tiles from blockIdx.x;
+    // TC_EPI_TRAIL: the first trailing row, the step's k-blocks and its
+    // units (blockIdx.y), tiles from blockIdx.x;
     // trail_lower: only tiles reaching the diagonal or below it (the
     // Hermitian factor), the others leave at once
-    int32_t c0;
+    int32_t r0, kblocks;
     const TcTrailUnit *trail;
     int32_t trail_lower;
     // limit of every mbarrier wait (0: TC_WAIT_NS, 2 s)
@@ -100,6 +104,7 @@ struct TcGramPlan {
 // trailing block has at least min_m rows.  Each unit owns operand rows in
 // the stacks sized for its first step; later steps reuse them.
 struct TcTrailPlan {
+    int parts = 1;                   // 32-column panels per step
     std::vector<TcTrailUnit> units;  // every step's units, concatenated
     std::vector<int32_t> u_off;      // per step: first entry (steps + 1 values)
     std::vector<int32_t> max_tiles, max_mpad, max_n2pad;  // per step
@@ -111,14 +116,20 @@ struct TcTrailPlan {
     int active(int step) const { return step < steps() ? u_off[step + 1] - u_off[step] : 0; }
 };
 cudaError_t tc_trail_plan(const std::vector<int> &s_desc, const std::vector<int32_t> &order, int n, int min_m,
-                          TcTrailPlan &p);
+                          int parts, TcTrailPlan &p);
 bool tc_trail_maps(TcTrailPlan &p, const float *hi, const float *lo);
-// Step `step` (c0 = 32 step): split L21 / U12 of the step's first `count`
+// Steps of several parts: units per step, and whether the device has the
+// shared memory their kernel takes (asked at planning).
+constexpr int TC_WIDE_MAX_UNITS = 16;
+bool tc_wide_ready();
+// Step `step` (c0 = 32 parts step): split L21 / U12 of the step's first `count`
 // units (<= active(step)) into the stacks, then the GEMM subtracting
 // L21 U12 from each one's A22.
 // lower: the Hermitian factor's update, tiles on and below the diagonal
 // only; persistent: one CTA per SM over the step's tiles with the
-// accumulator double-buffered in TMEM (else one 128 x 64 tile per CTA)
+// accumulator double-buffered in TMEM (else one 128 x 64 tile per CTA).
+// Steps of several parts run 128 x 128 tiles: at K = 256 the operands'
+// L2 traffic, not the read-modify-write of A22, is what a wider tile saves.
 cudaError_t tc_trail_run(const TcTrailPlan &p, int step, int count, const TcTrailUnit *d_trail, const UnitDesc *d_systems,
                          const MixedUnit *d_smu, float2 *a32, float *hi, float *lo, int32_t *status, cudaStream_t st,
                          bool lower = false, bool persistent = true);

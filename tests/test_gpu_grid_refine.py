@@ -1,6 +1,7 @@
-"""The grid-wide refinement at the edges of its 256-row diagonal blocks:
-meshes whose S is just above a multiple of 256 or below one, against the
-plain FP64 form (Zin 1e-6, currents 1e-7 normwise: the mixed form's gates)."""
+"""The grid-wide refinement at the edges of its 256-row diagonal blocks, and
+the factor's 128-column steps at the edges of theirs (S of 3,072 and above):
+meshes whose S is just above a multiple of the width or below one, against
+the plain FP64 form (Zin 1e-6, currents 1e-7 normwise: the mixed form's gates)."""
 import numpy as np
 import pytest
 
@@ -17,9 +18,10 @@ def acc():
 
 
 # a grid of nx x ny cells has 3 (nx (ny + 1) + ny (nx + 1)) unknowns
-@pytest.mark.parametrize("edges,pivoting", [(512, 0), (513, 0), (597, 0), (598, 1), (683, 0), (720, 1)])
+@pytest.mark.parametrize("edges,pivoting", [(512, 0), (513, 0), (597, 0), (598, 1), (683, 0), (720, 1), (1023, 0),
+                                            (1024, 0), (1025, 0), (1066, 0), (1067, 0), (1109, 0), (1109, 1)])
 def test_mixed_mesh_matches_plain(acc, edges, pivoting):
-    w, s, f = bench.mesh_workload(19)
+    w, s, f = bench.mesh_workload(24)
     ant = acc.Antenna(acc.wires_array(w[:edges]), acc.sources_array([(7, 1, 1.0)]), [f], 1)
     plain = acc.HallenBatch([ant]).solve()
     b = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
@@ -31,3 +33,16 @@ def test_mixed_mesh_matches_plain(acc, edges, pivoting):
     assert np.linalg.norm(x1 - x0) <= 1e-7 * np.linalg.norm(x0)
     z0, z1 = (complex(r.feeds[0][0][5], r.feeds[0][0][6]) for r in (plain, mixed))
     assert abs(z1 - z0) <= 1e-6 * abs(z0)
+
+
+def test_wide_steps_of_several_units_beside_small_ones(acc):
+    """Two systems that take 128-column steps (one a multiple of 128 tall),
+    a mid-size and a small one in one batch: each equals its own solve."""
+    w, s, f = bench.mesh_workload(24)
+    ants = [acc.Antenna(acc.wires_array(w[:e]), acc.sources_array([(7, 1, 1.0)]), [f], 1) for e in (1024, 300, 1040, 40)]
+    both = acc.HallenBatch(ants, precision=acc.PRECISION_MIXED).solve()
+    for u, ant in enumerate(ants):
+        alone = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED).solve()
+        assert both.status[u] == 0 and alone.status[0] == 0
+        x0, x1 = alone.currents[0], both.currents[u]
+        assert np.linalg.norm(x1 - x0) <= 1e-7 * np.linalg.norm(x0)
