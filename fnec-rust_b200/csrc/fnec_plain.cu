@@ -1124,62 +1124,67 @@ __global__ void __launch_bounds__(4 * SU_COLS) k_swap_u12(const UnitDesc *__rest
 constexpr size_t SU_SMEM = sizeof(cx) * (2 * NB * SU_LD + NB * (NB + 1));
 
 // A22 -= L21 * U12 with per-element in-order accumulation over the panel.
-// grid.x = tiles of 64x64 over the trailing block, grid.y = unit.
+// grid.x = tiles of TT x TT over the trailing block, grid.y = unit.
+// 32 wide, as the Gram's tiles, for their raggedness and the number of CTAs;
+// the panel blocks stage by cp.async beside the tile's own loads.  Measured,
+// factor phase, against 64 x 64 tiles staged first: one N = 255 system 0.65
+// -> 0.57 ms, 512 random antennas 10.4 -> 9.4, 20 x 20 mesh 11.4 -> 10.9,
+// 30 x 30 (S = 5580) 55.0 -> 55.4.
+constexpr int TT = 32;
 __global__ void __launch_bounds__(256) k_trailing(const UnitDesc *__restrict__ units, int c0,
                                                   cx *abuf, const int32_t *__restrict__ status, const int32_t *__restrict__ order, int base) {
-    extern __shared__ cx s_dyn[];
-    cx(*s_l)[NB + 1] = reinterpret_cast<cx(*)[NB + 1]>(s_dyn);
-    cx(*s_u)[64] = reinterpret_cast<cx(*)[64]>(s_dyn + 64 * (NB + 1));
+    constexpr int P = TT / 16;
+    __shared__ cx s_l[TT][NB + 1];
+    __shared__ cx s_u[NB][TT];
     int ui = order[base + blockIdx.y];
     UnitDesc u = units[ui];
     int s = u.s;
     if (c0 + NB >= s || status[ui] != 0) return;  // no trailing block (or a failed unit)
     int r0 = c0 + NB;  // first trailing row/column
     int rows = s - r0, cols = s + 1 - r0;
-    int tiles_c = (cols + 63) / 64;
-    int tiles_r = (rows + 63) / 64;
+    int tiles_c = (cols + TT - 1) / TT;
+    int tiles_r = (rows + TT - 1) / TT;
     int tile = blockIdx.x;
     if (tile >= tiles_r * tiles_c) return;
-    int R0 = r0 + (tile / tiles_c) * 64;
-    int K0 = r0 + (tile % tiles_c) * 64;
+    int R0 = r0 + (tile / tiles_c) * TT;
+    int K0 = r0 + (tile % tiles_c) * TT;
     int w1 = s + 1;
     cx *A = abuf + u.a_off;
     int tid = threadIdx.x;
-    for (int e = tid; e < 64 * NB; e += 256) {
-        int rr = e / NB, q = e % NB;
-        int R = R0 + rr;
-        s_l[rr][q] = (R < s) ? A[(int64_t)R * w1 + c0 + q] : cx_make(0.0, 0.0);
-    }
-    for (int e = tid; e < NB * 64; e += 256) {
-        int q = e / 64, cc = e % 64;
-        int K = K0 + cc;
-        s_u[q][cc] = (K <= s) ? A[(int64_t)(c0 + q) * w1 + K] : cx_make(0.0, 0.0);
-    }
-    __syncthreads();
     int ty = tid / 16, tx = tid % 16;
-    cx acc[4][4];
+    // the panel blocks stage while the tile's own entries load; rows and
+    // columns past the end repeat the last one and are not written back
+    for (int e = tid; e < TT * NB; e += 256)
+        cp_async_cx(&s_l[e / NB][e % NB], &A[(int64_t)min(R0 + e / NB, s - 1) * w1 + c0 + e % NB]);
+    for (int e = tid; e < NB * TT; e += 256)
+        cp_async_cx(&s_u[e / TT][e % TT], &A[(int64_t)(c0 + e / TT) * w1 + min(K0 + e % TT, s)]);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    cx acc[P][P];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < P; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < P; ++b) {
             int R = R0 + ty + 16 * a, K = K0 + tx + 16 * b;
             acc[a][b] = (R < s && K <= s) ? A[(int64_t)R * w1 + K] : cx_make(0.0, 0.0);
         }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll 4
     for (int q = 0; q < NB; ++q) {
-        cx lv[4], uv[4];
+        cx lv[P], uv[P];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) lv[a] = s_l[ty + 16 * a][q];
+        for (int a = 0; a < P; ++a) lv[a] = s_l[ty + 16 * a][q];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) uv[b] = s_u[q][tx + 16 * b];
+        for (int b = 0; b < P; ++b) uv[b] = s_u[q][tx + 16 * b];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < P; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = cx_sub(acc[a][b], cx_mul(lv[a], uv[b]));
+            for (int b = 0; b < P; ++b) acc[a][b] = cx_sub(acc[a][b], cx_mul(lv[a], uv[b]));
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < P; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < P; ++b) {
             int R = R0 + ty + 16 * a, K = K0 + tx + 16 * b;
             if (R < s && K <= s) A[(int64_t)R * w1 + K] = acc[a][b];
         }
@@ -1773,7 +1778,6 @@ void launch_gram_exact(const UnitDesc *units, int nu, int max_w, const AntDesc *
         k_gram_finish<<<nu, 256, 0, st>>>(units, ants, cons, codes, A);
     }
 }
-constexpr size_t TRAILING_SMEM = sizeof(cx) * (64 * (NB + 1) + NB * 64);
 
 // Raises a kernel's dynamic shared-memory limit once per device: the
 // attribute belongs to the kernel in the current device's context, so a
@@ -1892,8 +1896,7 @@ static void launch_panel_cluster(const UnitDesc *units, int n, int m_max, int c0
 uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const GridPlan &gp, cx *A,
                              int32_t *piv, int32_t *status, cudaStream_t st) {
     uint64_t L = 0;
-    set_smem_limit_once(k_trailing, (int)TRAILING_SMEM);  // once per device
-    set_smem_limit_once(k_swap_u12, (int)SU_SMEM);
+    set_smem_limit_once(k_swap_u12, (int)SU_SMEM);  // once per device
     set_smem_limit_once(k_panel_cluster<false>, (int)cp_smem(CP_MAX_ROWS));
     set_smem_limit_once(k_panel_cluster<true>, (int)cp_smem(CP_MAX_ROWS));
     set_smem_limit_once(k_panel_grid, 96 * 1024);
@@ -1940,9 +1943,9 @@ uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const Gri
             ++L;
             int rows = m - NB;
             if (rows > 0) {
-                int t = ((rows + 63) / 64) * ((rest + 63) / 64);
+                int t = ((rows + TT - 1) / TT) * ((rest + TT - 1) / TT);
                 dim3 g2(t, c.i1 - c.i0);
-                k_trailing<<<g2, 256, TRAILING_SMEM, st>>>(units, c0, A, status, ord, c.i0);
+                k_trailing<<<g2, 256, 0, st>>>(units, c0, A, status, ord, c.i0);
                 ++L;
             }
         }
