@@ -2715,6 +2715,18 @@ int fnec_batch_read_z(fnec_batch *b, uint32_t unit, double *z) {
 
 // ---- reference nec_accel entry points ---------------------------------------
 
+// Device memory of one call, from the device's stream-ordered pool on the
+// context's stream (cudaMalloc and cudaFree cost a one-call entry most of a
+// millisecond, and stall every stream of the device).
+struct CallMemory {
+    cudaStream_t st;
+    void *p = nullptr;
+    cudaError_t alloc(size_t bytes) { return cudaMallocAsync(&p, bytes, st); }
+    ~CallMemory() {
+        if (p) cudaFreeAsync(p, st);
+    }
+};
+
 int fnec_fill_zmatrix(fnec_ctx *ctx, const fnec_zsegment *segments, uint64_t n, double freq_hz,
                       int32_t ground, double *z_out) {
     if (!ctx || (!segments && n) || (!z_out && n)) return FNEC_ERR_BAD_ARG;
@@ -2733,14 +2745,15 @@ int fnec_fill_zmatrix(fnec_ctx *ctx, const fnec_zsegment *segments, uint64_t n, 
         s.self_log = self_log_term(s.len, s.rad);
         hs[i] = s;
     }
-    DevSeg *d_s = nullptr;
-    cx *d_z = nullptr;
-    CUDA_TRY(ctx, cudaMalloc(&d_s, sizeof(DevSeg) * n));
-    cudaError_t e = cudaMalloc(&d_z, sizeof(cx) * n * n);
+    CallMemory m_s{ctx->stream}, m_z{ctx->stream};
+    CUDA_TRY(ctx, m_s.alloc(sizeof(DevSeg) * n));
+    cudaError_t e = m_z.alloc(sizeof(cx) * n * n);
     if (e != cudaSuccess) {
-        cudaFree(d_s);
+        (void)cudaGetLastError();
         return fail(ctx, FNEC_ERR_OUT_OF_MEMORY, "fill_zmatrix: Z allocation");
     }
+    DevSeg *d_s = static_cast<DevSeg *>(m_s.p);
+    cx *d_z = static_cast<cx *>(m_z.p);
     e = cudaMemcpyAsync(d_s, hs.data(), sizeof(DevSeg) * n, cudaMemcpyHostToDevice, ctx->stream);
     double k = 2.0 * PI * freq_hz / C0;
     if (e == cudaSuccess) {
@@ -2750,8 +2763,6 @@ int fnec_fill_zmatrix(fnec_ctx *ctx, const fnec_zsegment *segments, uint64_t n, 
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(z_out, d_z, sizeof(cx) * n * n, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(d_s);
-    cudaFree(d_z);
     if (e != cudaSuccess) return fail(ctx, FNEC_ERR_CUDA, cudaGetErrorString(e));
     return FNEC_OK;
 }
@@ -2991,8 +3002,9 @@ int fnec_near_field(fnec_ctx *ctx, const fnec_gpu_segment *segments, uint64_t n,
     cudaSetDevice(ctx->device);
     const size_t n_seg = 7 * n, n_cur = 2 * n, n_pts = 3 * p, n_fld = 6 * p;
     const size_t total = n_seg + n_cur + n_pts + (e_out ? n_fld : 0) + (h_out ? n_fld : 0);
-    double *d = nullptr;
-    CUDA_TRY(ctx, cudaMalloc(&d, sizeof(double) * total));
+    CallMemory mem{ctx->stream};
+    CUDA_TRY(ctx, mem.alloc(sizeof(double) * total));
+    double *d = static_cast<double *>(mem.p);
     double *d_seg = d, *d_cur = d_seg + n_seg, *d_pts = d_cur + n_cur, *d_e = d_pts + n_pts;
     double *d_h = d_e + (e_out ? n_fld : 0);
     cudaStream_t s = ctx->stream;
@@ -3009,7 +3021,6 @@ int fnec_near_field(fnec_ctx *ctx, const fnec_gpu_segment *segments, uint64_t n,
     if (e == cudaSuccess && e_out) e = cudaMemcpyAsync(e_out, d_e, sizeof(double) * n_fld, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && h_out) e = cudaMemcpyAsync(h_out, d_h, sizeof(double) * n_fld, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d);
     if (e != cudaSuccess) return fail(ctx, FNEC_ERR_CUDA, cudaGetErrorString(e));
     return FNEC_OK;
 }
