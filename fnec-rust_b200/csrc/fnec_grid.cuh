@@ -44,35 +44,46 @@ __device__ __forceinline__ unsigned long long gtimer_ns() {
 // before the launch; nblocks CTAs take part; each CTA waits at most wait_ns.
 // Returns false (in every thread of the CTA) when the barrier failed: the
 // caller returns at once.
-__device__ __forceinline__ bool grid_barrier(GridSync *gs, unsigned int nblocks, unsigned int epoch,
-                                             unsigned long long wait_ns = GRID_WAIT_NS) {
+// It is an arrival (the CTA's writes before it are released) and a wait (the
+// others' are acquired); between the two a CTA may do work no other waits for.
+__device__ __forceinline__ void grid_arrive(GridSync *gs) {
+    __syncthreads();  // orders the CTA's writes before thread 0's release
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gs->count) : "memory");
+}
+__device__ __forceinline__ bool grid_wait(GridSync *gs, unsigned int nblocks, unsigned int epoch,
+                                          unsigned long long wait_ns = GRID_WAIT_NS) {
     __shared__ int s_ok;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&gs->count, 1u);
         const unsigned int target = epoch * nblocks;
-        volatile unsigned int *cnt = &gs->count;
-        volatile int *err = &gs->err;
         int ok = 1;
-        unsigned long long t0 = gtimer_ns();
-        while (*cnt < target) {
-            if (*err) {
+        unsigned long long t0 = 0;
+        for (unsigned int it = 0;; ++it) {
+            unsigned int cnt;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cnt) : "l"(&gs->count) : "memory");
+            if (cnt >= target) break;
+            if ((it & 31) != 31) continue;  // the clock and the error word are looked at now and then
+            if (*(volatile int *)&gs->err) {
                 ok = 0;
                 break;
             }
-            if (gtimer_ns() - t0 > wait_ns) {
+            const unsigned long long now = gtimer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > wait_ns) {
                 atomicExch(&gs->err, 1);
                 ok = 0;
                 break;
             }
-            __nanosleep(64);
         }
         __threadfence();
         s_ok = ok;
     }
     __syncthreads();
     return s_ok != 0;
+}
+__device__ __forceinline__ bool grid_barrier(GridSync *gs, unsigned int nblocks, unsigned int epoch,
+                                             unsigned long long wait_ns = GRID_WAIT_NS) {
+    grid_arrive(gs);
+    return grid_wait(gs, nblocks, epoch, wait_ns);
 }
 
 // Exchange area of one unit's grid panel: per CTA its pivot candidate and

@@ -2094,34 +2094,72 @@ __device__ bool gg_apply(GGrid &c, const cx *v, cx *out) {
 }
 
 // y[r] -= sum_q lu[r][c0 + q] x[q] for rows r0 <= r < r1, x the nb solved
-// entries in shared memory: a warp per row, a row's segment 8 loads a lane.
-__device__ __forceinline__ void gg_update(GGrid &c, cx *y, const cx *sx, int r0, int r1, int c0, int nb) {
+// entries in shared memory: a warp takes R rows at a time, 8 R loads a lane
+// in flight.  The bytes in flight bound it: refinement of the 46 x 46 mesh
+// 27.8 ms with one row at a time, 22.4 with two, 17.2 with six (19.3 with
+// eight; the factor copied into blocks of GI columns, so that a step's rows
+// follow each other in memory, changes nothing).  Two rows where a step has
+// no more per warp: 20 x 20 mesh 2.24 ms against 2.41.
+template <int R>
+__device__ __forceinline__ void gg_update_rows(GGrid &c, cx *y, const cx *sx, int r0, int r1, int c0, int nb) {
     const GmresCtx &g = c.g;
-    for (int r = r0 + c.gw; r < r1; r += c.TW) {
-        const float2 *row = g.lu + (int64_t)r * g.s + c0;
-        float2 l[GI / 32];
+    constexpr int Q = GI / 32;
+    for (int rb = r0 + c.gw; rb < r1; rb += R * c.TW) {
+        float2 l[R][Q];
+        cx yr[R];
 #pragma unroll
-        for (int q = 0; q < GI / 32; ++q) l[q] = c.lane + 32 * q < nb ? row[c.lane + 32 * q] : cf(0.f, 0.f);
-        const cx yr = ldcg_cx(y + r);
-        cx acc = {0, 0};
+        for (int j = 0; j < R; ++j) {
+            const int r = min(rb + j * c.TW, r1 - 1);
+            const float2 *row = g.lu + (int64_t)r * g.s + c0;
 #pragma unroll
-        for (int q = 0; q < GI / 32; ++q) acc = zadd(acc, zmul(f2z(l[q]), sx[c.lane + 32 * q]));
-        acc = warp_sum(acc);
-        if (c.lane == 0) y[r] = zsub(yr, acc);
+            for (int q = 0; q < Q; ++q) l[j][q] = c.lane + 32 * q < nb ? row[c.lane + 32 * q] : cf(0.f, 0.f);
+            yr[j] = ldcg_cx(y + r);
+        }
+        cx acc[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[j] = {0, 0};
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const cx x = sx[c.lane + 32 * q];
+#pragma unroll
+            for (int j = 0; j < R; ++j) acc[j] = zadd(acc[j], zmul(f2z(l[j][q]), x));
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[j] = warp_sum(acc[j]);
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (c.lane == 0 && rb + j * c.TW < r1) y[rb + j * c.TW] = zsub(yr[j], acc[j]);
     }
 }
 
-// x = inv y for one diagonal block (lower: columns up to the row, else from it)
-__device__ __forceinline__ void gg_block_solve(GGrid &c, const cx *inv, const cx *y, cx *x, int nb, bool lower) {
-    for (int i = c.gw; i < nb; i += c.TW) {
-        const cx *row = inv + (int64_t)i * GI;
-        cx acc = {0, 0};
-        const int b = lower ? 0 : (i & ~31), e = lower ? i + 1 : nb;
-        for (int q = b + c.lane; q < e; q += 32)
-            if (q >= (lower ? 0 : i)) acc = zadd(acc, zmul(row[q], ldcg_cx(y + q)));
-        acc = warp_sum(acc);
-        if (c.lane == 0) x[i] = acc;
+__device__ __forceinline__ void gg_update(GGrid &c, cx *y, const cx *sx, int r0, int r1, int c0, int nb) {
+    if (r1 - r0 > 2 * c.TW) gg_update_rows<6>(c, y, sx, r0, r1, c0, nb);
+    else gg_update_rows<2>(c, y, sx, r0, r1, c0, nb);
+}
+
+// x = inv y for one diagonal block (lower: columns up to the row, else from
+// it), its rows dealt over the CTAs; row: the warp's entries of the inverse,
+// loaded ahead by gg_block_row
+__device__ __forceinline__ int gg_block_index(const GGrid &c) { return c.wid * c.G + c.cta; }
+__device__ __forceinline__ void gg_block_row(const GGrid &c, const cx *inv, int nb, bool lower, cx (&row)[GI / 32]) {
+    const int i = gg_block_index(c);
+#pragma unroll
+    for (int q = 0; q < GI / 32; ++q) {
+        const int k = c.lane + 32 * q;
+        const bool in = i < nb && (lower ? k <= i : k >= i && k < nb);
+        row[q] = in ? inv[(int64_t)i * GI + k] : cx{0, 0};
     }
+}
+__device__ __forceinline__ void gg_block_solve(const GGrid &c, const cx (&row)[GI / 32], const cx *y, cx *x, int nb) {
+    const int i = gg_block_index(c);
+    if (i >= nb) return;
+    cx v[GI / 32], acc = {0, 0};
+#pragma unroll
+    for (int q = 0; q < GI / 32; ++q) v[q] = c.lane + 32 * q < nb ? ldcg_cx(y + c.lane + 32 * q) : cx{0, 0};
+#pragma unroll
+    for (int q = 0; q < GI / 32; ++q) acc = zadd(acc, zmul(row[q], v[q]));
+    acc = warp_sum(acc);
+    if (c.lane == 0) x[i] = acc;
 }
 
 // out = (L U)^-1 P in through the diagonal blocks' inverses: a block's
@@ -2132,20 +2170,28 @@ __device__ __forceinline__ void gg_block_solve(GGrid &c, const cx *inv, const cx
 // bounded the whole refinement.  The inverses are FP64, so this is the same
 // operator to FP64 rounding (results agree to 2e-14).  GI: at 256 a block's
 // inverse adds 4 KB a row to the 2 x 8 S bytes of the factor's.
-// Measured, refinement phase: 46 x 46 mesh (S = 12,972) 67.9 -> 21.0 ms,
-// 20 x 20 (S = 2520) 8.15 -> 2.28 ms, 16 x 16 (S = 1632) 5.0 -> 1.5 ms.
+// Measured, refinement phase: 46 x 46 mesh (S = 12,972) 67.9 -> 17.2 ms,
+// 20 x 20 (S = 2520) 8.15 -> 2.24 ms, 16 x 16 (S = 1632) 5.0 -> 1.5 ms.
 __device__ bool gg_prec_inv(GGrid &c, const cx *in, cx *out) {
     const int s = c.g.s, nblk = (s + GI - 1) / GI;
     __shared__ cx s_x[GI];
     for (int i = c.gt; i < s; i += c.T) c.y[i] = ldcg_cx(in + c.perm[i]);
     GG_SYNC(c);
+    cx row[GI / 32];
+    gg_block_row(c, c.inv, min(GI, s), true, row);
     for (int dir = 0; dir < 2; ++dir) {  // forward y -> y2, then backward y2 -> y
         cx *y = dir ? c.y2 : c.y, *x = dir ? c.y : c.y2;
         for (int t = 0; t < nblk; ++t) {
             const int bk = dir ? nblk - 1 - t : t, c0 = bk * GI, nb = min(GI, s - c0);
-            gg_block_solve(c, c.inv + ((int64_t)bk * 2 + dir) * GI * GI, y + c0, x + c0, nb, dir == 0);
+            gg_block_solve(c, row, y + c0, x + c0, nb);
+            // the next block's inverse: nothing below writes it
+            const bool last = t + 1 == nblk, low = dir == 0 && !last;
+            if (dir == 0 || !last) {
+                const int nx = last ? bk : (dir ? bk - 1 : bk + 1);
+                gg_block_row(c, c.inv + ((int64_t)nx * 2 + !low) * GI * GI, min(GI, s - nx * GI), low, row);
+            }
             GG_SYNC(c);
-            if (t + 1 == nblk) break;
+            if (last) break;
             for (int i = c.tid; i < GI; i += blockDim.x) s_x[i] = i < nb ? ldcg_cx(x + c0 + i) : cx{0, 0};
             __syncthreads();
             if (dir == 0) gg_update(c, y, s_x, c0 + nb, s, c0, nb);
@@ -2439,7 +2485,7 @@ __device__ bool gmres_grid_body(GGrid &c, const UnitDesc &u, MixedUnit *mus, int
     return true;
 }
 
-__global__ void __launch_bounds__(256) k_gmres_grid(const UnitDesc *__restrict__ units, const AntDesc *__restrict__ ants,
+__global__ void __launch_bounds__(256, 1) k_gmres_grid(const UnitDesc *__restrict__ units, const AntDesc *__restrict__ ants,
                                                     MixedUnit *mus, int ui, const int32_t *__restrict__ ibuf,
                                                     const DevConRow *__restrict__ crows, const cx *__restrict__ zbuf,
                                                     const cx *__restrict__ rhs, const double *__restrict__ cosv,
