@@ -97,7 +97,8 @@ __device__ __forceinline__ cx elem_fast(const double *om, const double *od, cons
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             double l = m_gl_n4[m] * half;
-            double r = sqrt(l * l + a * a);
+            double r = sqrt(fma(l, l, __dmul_rn(a, a)));  // written out: the self term's bits
+                                                          // stay with any contraction
             double sn, cs;
             sincos(-k * r, &sn, &cs);
             double inv = 1.0 / r;
@@ -106,7 +107,7 @@ __device__ __forceinline__ cx elem_fast(const double *om, const double *od, cons
         }
         ire *= half;
         iim *= half;
-        double r_end = sqrt(half * half + a * a);
+        double r_end = sqrt(fma(half, half, __dmul_rn(a, a)));
         ire += 2.0 * log((half + r_end) / a);
     } else {
         const double kpi = k * 0.31830988618379067;  // k / pi
