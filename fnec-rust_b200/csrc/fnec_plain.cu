@@ -1202,8 +1202,9 @@ __global__ void __launch_bounds__(256) k_trailing(const UnitDesc *__restrict__ u
 // new when the row begins.  One barrier per piece.
 // Measured, 20 x 20 mesh (S = 2520, 3.2 M subtractions): 48.4 ms with one
 // warp that formed and shuffled the products between the subtractions (30
-// cycles each) -> 17.3 ms (10.6 cycles; a dependent double add takes 8.2).
-// 512 random antennas (S up to 700): 3.47 -> 1.12 ms.
+// cycles each) -> 15.9 ms (9.8 cycles; a dependent double add takes 8.2;
+// 17.3 with the subtractions in loops of 16 instead of 64).
+// 512 random antennas (S up to 700): 3.47 -> 1.06 ms.
 // x may alias b (b_in_x: b is read from x): b_i is read before x_i is
 // written, and only x_j, j > i, is read after.
 constexpr int BP = 256;          // products per piece: 2,000+ cycles of chain per barrier
@@ -1281,16 +1282,25 @@ __device__ __forceinline__ void backsub_rows(const cx *A, int s, int w1, const c
 #pragma unroll
                 for (int q = 0; q < 8; ++q) p[q] = q8[q];
             };
-            read8(p0, 0);
-#pragma unroll 1
-            for (int e = 0; e < cnt; e += 16) {
+            auto sub16 = [&](int e) {
                 read8(p1, e + 8);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) sum = cx_sub(sum, p0[q]);
                 read8(p0, e + 16);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) sum = cx_sub(sum, p1[q]);
+            };
+            read8(p0, 0);
+            int e = 0;
+#pragma unroll 1
+            for (; e + 64 <= cnt; e += 64) {
+                sub16(e);
+                sub16(e + 16);
+                sub16(e + 32);
+                sub16(e + 48);
             }
+#pragma unroll 1
+            for (; e < cnt; e += 16) sub16(e);
             if (cur.j0 + BP >= s) {
                 x_prev = cx_div(sum, diag);
                 if (tid == 0) xs[cur.i] = x_prev;
