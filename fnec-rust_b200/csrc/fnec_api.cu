@@ -3125,6 +3125,7 @@ struct ServerReq {
     fnec_request_out out{};
     bool copy_out = false;
     int64_t bytes = 0;
+    bool large = false;  // bytes holds the large systems' own scratch
     uint32_t n_solves = 0, n = 0, s = 0, n_points = 0, n_feed_rows = 0;
     Clock::time_point t_submit, t_done;
     int32_t state = FNEC_REQ_QUEUED;
@@ -3144,7 +3145,9 @@ struct Lane {
 
 // Upper bound of the device bytes one request's batch needs (Z, the
 // factor, solution and work vectors, Gram operand stacks, pattern buffers).
-int64_t request_bytes(const HostAnt &h, int precision) {
+// large: with the scratch that only a batch planned with allow_grid takes
+// (the wide factor steps', the grid-wide refinement's block inverses).
+int64_t request_bytes(const HostAnt &h, int precision, bool large = true) {
     const int64_t n = (int64_t)h.segs.size(), w = h.cols(), s = n + w;
     const int64_t f = (int64_t)h.freqs.size(), r = (int64_t)std::max<size_t>(h.rhs_srcs.size(), 1);
     const int64_t rows = n + 2 * w + (int64_t)h.ja.size();
@@ -3169,14 +3172,15 @@ int64_t request_bytes(const HostAnt &h, int precision) {
         if (s - 32 >= 192) {                               // tensor-core trailing stacks and step lists
             const int64_t m0 = s - 32, pa = (m0 + 127) / 128 * 128, pb = (2 * m0 + 127) / 128 * 128;
             b += (256 * (2 * pa + 2 * pb) + 32 * ((s + 31) / 32)) * f;
-            if (s >= 3072) b += (2048 * (pa + pb) + 64 * ((s + 127) / 128) + 1024) * f;  // wide factor steps
+            if (large && s >= 3072) b += (2048 * (pa + pb) + 64 * ((s + 127) / 128) + 1024) * f;  // wide factor steps
         }
     } else {
         b += 16 * s * (s + 1) * f + 4 * s * f;             // FP64 factor, pivots
     }
     if (s > 380) b += (int64_t)grid_xchg_bytes() + (int64_t)grid_sync_bytes((int)((s + 31) / 32));  // grid panels
     if (precision == FNEC_PRECISION_MIXED && s >= 1536)   // grid-wide GMRES scratch
-        b += 16 * n * ((n + 255) / 256) + 96 * s + 16 * 2 * 256 * (s + 256) + 16 * 2 * 296 * 25 + 8192;
+        b += 16 * n * ((n + 255) / 256) + 64 * s + 16 * 2 * 296 * 25 + 4096 +
+             (large ? 32 * s + 16 * 2 * 256 * (s + 256) + 4096 : 0);
     return b + (1 << 20);
 }
 
@@ -3330,11 +3334,15 @@ void lane_worker(fnec_server *S, Lane *L) {
         }
         std::vector<HostAnt> hs;
         hs.reserve(take.size());
-        for (ServerReq *r : take) hs.push_back(r->host);
+        bool large = S->lanes.size() == 1;  // cooperative kernels need the whole device
+        for (ServerReq *r : take) {
+            hs.push_back(r->host);
+            large = large && r->large;
+        }
         BatchPlace place;
         place.st = L->st;
         place.pooled = true;
-        place.allow_grid = S->lanes.size() == 1;  // cooperative kernels need the whole device
+        place.allow_grid = large;
         place.in = &L->in;
         place.out = &slab->mem;
         place.aux = &L->aux;
@@ -3550,7 +3558,11 @@ int fnec_server_submit(fnec_server *S, const fnec_antenna *req, const fnec_reque
     for (auto &v : h.rhs_feeds) fr += (uint32_t)v.size();
     r->n_feed_rows = fr * (uint32_t)h.freqs.size();
     r->status.assign(r->n_solves, 0);
-    r->bytes = request_bytes(h, S->cfg.precision);
+    // a request whose large systems' scratch would not fit the budget, or
+    // whose lane could not use it, is planned and counted without it
+    const int64_t full = request_bytes(h, S->cfg.precision);
+    r->large = S->lanes.size() == 1 && full <= (int64_t)S->cfg.hbm_budget_bytes;
+    r->bytes = r->large ? full : request_bytes(h, S->cfg.precision, false);
     if (info) {
         info->n_segments = r->n;
         info->n_rhs = (uint32_t)std::max<size_t>(h.rhs_srcs.size(), 1);
@@ -3558,7 +3570,7 @@ int fnec_server_submit(fnec_server *S, const fnec_antenna *req, const fnec_reque
         info->n_feed_rows = r->n_feed_rows;
         info->n_points = r->n_points;
         info->pad = 0;
-        info->device_bytes = (uint64_t)r->bytes;
+        info->device_bytes = (uint64_t)full;
     }
     if (r->bytes > (int64_t)S->cfg.hbm_budget_bytes) {
         delete r;

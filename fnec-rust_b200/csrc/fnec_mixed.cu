@@ -2892,27 +2892,36 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
                b_sync = sizeof(GridSync) * w.grid_solves.size();
         size_t gt = al(b_perm) + al(b_part) + 2 * al(b_y) + al(b_inv) + al(b_red) + al(b_sync);
         e = dev.alloc(&w.grid_base, gt);
+        if (e == cudaErrorMemoryAllocation) {  // no room for it: these solves refine in one CTA each
+            (void)cudaGetLastError();
+            w.grid_base = nullptr;
+            w.grid_solves.clear();
+            w.grid_s.clear();
+            e = cudaSuccess;
+        }
         if (e != cudaSuccess) return e;
-        unsigned char *q = (unsigned char *)w.grid_base;
-        w.g_perm = (int32_t *)q;
-        q += al(b_perm);
-        w.g_part = (cx *)q;
-        q += al(b_part);
-        w.g_y = (cx *)q;
-        q += al(b_y);
-        w.g_y2 = (cx *)q;
-        q += al(b_y);
-        w.g_inv = (cx *)q;
-        q += al(b_inv);
-        w.g_red = (cx *)q;
-        q += al(b_red);
-        w.g_sync = q;
-        w.bytes += gt;
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 256, 0);
-        w.grid_ctas = std::min(GG_MAX_CTAS, sms * std::min(per_sm, 1));
+        if (w.grid_base) {
+            unsigned char *q = (unsigned char *)w.grid_base;
+            w.g_perm = (int32_t *)q;
+            q += al(b_perm);
+            w.g_part = (cx *)q;
+            q += al(b_part);
+            w.g_y = (cx *)q;
+            q += al(b_y);
+            w.g_y2 = (cx *)q;
+            q += al(b_y);
+            w.g_inv = (cx *)q;
+            q += al(b_inv);
+            w.g_red = (cx *)q;
+            q += al(b_red);
+            w.g_sync = q;
+            w.bytes += gt;
+            int dev = 0, sms = 0, per_sm = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 256, 0);
+            w.grid_ctas = std::min(GG_MAX_CTAS, sms * std::min(per_sm, 1));
+        }
     }
     {
         // cluster GMRES when one CTA per solve cannot fill the GPU
@@ -3020,30 +3029,39 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
         }
         int n_wide = 0;
         while (n_wide < (int)sd.size() && sd[n_wide] >= WIDE_MIN_S) ++n_wide;
-        if (n_wide > 0 && n_wide <= TC_WIDE_MAX_UNITS && w.tc && tc_wide_ready()) {
+        if (allow_grid && n_wide > 0 && n_wide <= TC_WIDE_MAX_UNITS && w.tc && tc_wide_ready()) {
             TcTrailPlan *p = new TcTrailPlan();
             tc_trail_plan(sd, ord, n_wide, 1, WIDE / MNB, *p);
             size_t b_st = sizeof(float) * 32 * (size_t)p->rows, b_u = sizeof(TcTrailUnit) * (p->units.size() + 1);
             size_t tot = 2 * al(b_st) + al(b_u);
             e = dev.alloc(&w.wide_base, tot);
+            if (e == cudaErrorMemoryAllocation) {  // no room for it: 32-column steps
+                (void)cudaGetLastError();
+                w.wide_base = nullptr;
+                delete p;
+                p = nullptr;
+                e = cudaSuccess;
+            }
             if (e != cudaSuccess) {
                 delete p;
                 return e;
             }
-            unsigned char *q = (unsigned char *)w.wide_base;
-            w.wd_hi = (float *)q;
-            q += al(b_st);
-            w.wd_lo = (float *)q;
-            q += al(b_st);
-            w.d_wide = q;
-            w.bytes += tot;
-            e = dev.upload(w.d_wide, p->units.data(), sizeof(TcTrailUnit) * p->units.size());
-            if (e != cudaSuccess || !tc_trail_maps(*p, w.wd_hi, w.wd_lo)) {
-                delete p;
-                return e != cudaSuccess ? e : cudaErrorNotSupported;
+            if (p) {
+                unsigned char *q = (unsigned char *)w.wide_base;
+                w.wd_hi = (float *)q;
+                q += al(b_st);
+                w.wd_lo = (float *)q;
+                q += al(b_st);
+                w.d_wide = q;
+                w.bytes += tot;
+                e = dev.upload(w.d_wide, p->units.data(), sizeof(TcTrailUnit) * p->units.size());
+                if (e != cudaSuccess || !tc_trail_maps(*p, w.wd_hi, w.wd_lo)) {
+                    delete p;
+                    return e != cudaSuccess ? e : cudaErrorNotSupported;
+                }
+                w.wide = p;
+                w.wide_n = n_wide;
             }
-            w.wide = p;
-            w.wide_n = n_wide;
         }
     }
     if (systems.size() >= 4 && !w.fmade) {  // concurrent factor groups

@@ -109,7 +109,9 @@ struct MixedMarks {
 
 bool mixed_available();
 // systems: one per factorisation; solves: one per right-hand side.
-// allow_grid: large solves may take the grid-wide (cooperative) GMRES
+// allow_grid: large solves may take the grid-wide (cooperative) GMRES and large
+// Hermitian systems the wide factor steps, each with its own scratch (without
+// room for it they take the paths of smaller systems)
 cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, const std::vector<UnitDesc> &solves,
                         const std::vector<AntDesc> &ants, int max_s, const DevAlloc &dev, bool allow_grid);
 void free_mixed(MixedWork &w, const DevAlloc &dev);

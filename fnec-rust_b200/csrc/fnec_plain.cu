@@ -14,14 +14,15 @@
 //   k_expand_segments  geometry.rs:710-754     one CTA per GW wire
 //   k_hallen_rhs       excitation.rs:119-244   one CTA per unit
 //   k_fill_exact       matrix.rs:186-331       16x16 tiles of Z, tile list
-//   k_gram_zz          linear.rs:765-780       64x64 tiles of Z^H [Z | y]
+//   k_gram_zz          linear.rs:765-780       32x32 tiles of Z^H [Z | y], upper triangle
 //   k_gram_ccols       linear.rs:765-780       the -cos(k s) columns (sparse)
 //   k_gram_finish      linear.rs:757-785       constraint rows, then +1e-8 I
-//   k_panel            linear.rs:1343-1370     NB columns, one CTA per unit
-//   k_panel_grid       linear.rs:1343-1370     NB columns of a tall panel, many CTAs
+//   k_panel_cluster    linear.rs:1343-1370     NB columns, a thread per row, up to 8 CTAs per unit
+//   k_panel            linear.rs:1343-1370     the same from global memory, one CTA per unit
+//   k_panel_grid       linear.rs:1343-1370     NB columns of a panel above 3,072 rows, many CTAs
 //   k_swap_u12         linear.rs:1358-1369     deferred swaps + U block row
-//   k_trailing         linear.rs:1362-1369     A22 -= L21 U12, 64x64 tiles
-//   k_backsub          linear.rs:1372-1381     one warp per unit
+//   k_trailing         linear.rs:1362-1369     A22 -= L21 U12, 32x32 tiles
+//   k_backsub          linear.rs:1372-1381     one CTA per unit: a chain warp, two product warps
 //   k_feedpoints       solve_session.rs:846-947
 #include <algorithm>
 #include <cstdio>

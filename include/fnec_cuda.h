@@ -673,9 +673,10 @@ int fnec_batch_resolve(fnec_batch *b);
  * under every schedule); the mixed form stays within its refinement
  * tolerance under every schedule. */
 typedef struct {
-    int32_t grid_panels;   /* 1: panels too tall for one CTA's shared memory are
-                              factored grid-wide (cooperative launch); 0: one CTA
-                              from global memory                                  */
+    int32_t grid_panels;   /* 1: panels too tall for one CTA's shared memory (mixed)
+                              or one cluster's registers (plain, above 3,072 rows)
+                              are factored grid-wide (cooperative launch); 0: one
+                              CTA from global memory                              */
     int32_t class_shift;   /* panel and trailing launches group units whose
                               remaining heights share a 2^class_shift size class
                               (1 or 2)                                            */
@@ -701,7 +702,8 @@ typedef struct {
                               tcgen05 (3xTF32, complex as one real GEMM of K 64;
                               for the Hermitian factor only the tiles on and
                               below the diagonal); 0 all as FP32 SIMT tiles, one
-                              pass per step; 2 (GEPP only) SIMT tiles once per
+                              pass per step, but up to 16 Hermitian systems
+                              of S >= 3072 in 128-column tcgen05 steps; 2 (GEPP only) SIMT tiles once per
                               two steps (the first step updates only the next
                               panel's columns)                                   */
     int32_t gmres_ctas_per_sm;/* mixed: 3 or 4 refinement CTAs per SM (the

@@ -46,3 +46,21 @@ def test_wide_steps_of_several_units_beside_small_ones(acc):
         assert both.status[u] == 0 and alone.status[0] == 0
         x0, x1 = alone.currents[0], both.currents[u]
         assert np.linalg.norm(x1 - x0) <= 1e-7 * np.linalg.norm(x0)
+
+
+def test_server_takes_a_large_request_whose_own_scratch_misses_the_budget(acc):
+    """A budget 4 MB below a request's estimate leaves no room for the block
+    inverses' scratch (8 KB per row of S = 1,632, 13 MB): the request is still
+    taken, planned without it, and its result is the batch's."""
+    w, s, f = bench.mesh_workload(16)
+    ant = acc.Antenna(acc.wires_array(w), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    ref = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED).solve()
+    with acc.Server(acc.PRECISION_MIXED, lanes=1, hbm_budget_bytes=1 << 30) as srv:
+        need = srv.shape(ant).device_bytes
+    with acc.Server(acc.PRECISION_MIXED, lanes=1, hbm_budget_bytes=need - (4 << 20)) as srv:
+        r = srv.submit(ant, copy_out=True)
+        srv.wait(r)
+        currents, _, _, status = r.result()
+        assert status[0] == 0
+        x0, x1 = np.ravel(ref.currents[0]), np.ravel(currents)
+        assert np.linalg.norm(x1 - x0) <= 1e-7 * np.linalg.norm(x0)
