@@ -20,6 +20,7 @@
 // few directions.  The error against the FP64 oracle is reported per unit
 // (iterations and final residual are kept for inspection).
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <climits>
 #include <vector>
@@ -1975,6 +1976,7 @@ constexpr int GG_RC = 256;           // rows per column-sum chunk of M^H t
 constexpr int GG_MIN_S = 1536;       // solves this large go grid-wide ...
 constexpr int GG_MAX_SOLVES = 16;    // ... when there are at most this many
 constexpr int GG_MAX_CTAS = 296;
+constexpr int GG_WARPS = 8;          // warps per CTA
 
 __device__ __forceinline__ cx ldcg_cx(const cx *p) {
     double2 d = __ldcg(reinterpret_cast<const double2 *>(p));
@@ -2486,7 +2488,7 @@ __device__ bool gmres_grid_body(GGrid &c, const UnitDesc &u, MixedUnit *mus, int
     return true;
 }
 
-__global__ void __launch_bounds__(256, 1) k_gmres_grid(const UnitDesc *__restrict__ units, const AntDesc *__restrict__ ants,
+__global__ void __launch_bounds__(32 * GG_WARPS, 1) k_gmres_grid(const UnitDesc *__restrict__ units, const AntDesc *__restrict__ ants,
                                                     MixedUnit *mus, int ui, const int32_t *__restrict__ ibuf,
                                                     const DevConRow *__restrict__ crows, const cx *__restrict__ zbuf,
                                                     const cx *__restrict__ rhs, const double *__restrict__ cosv,
@@ -2764,6 +2766,10 @@ __global__ void k_perm_from_piv(const UnitDesc *__restrict__ units, int ui, cons
 
 bool mixed_available() { return true; }
 
+// Test hook (fnec_test_limit_refinement_ctas): CTAs a grid-wide refinement
+// planned from now on may take, as on a device partition of so few SMs.
+static std::atomic<int> g_grid_ctas_limit{GG_MAX_CTAS};
+
 cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, const std::vector<UnitDesc> &solves,
                         const std::vector<AntDesc> &ants, int max_s, const DevAlloc &dev, bool allow_grid) {
     std::vector<int64_t> a32_of(systems.size()), binv_of(systems.size());
@@ -2919,8 +2925,8 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             int dev = 0, sms = 0, per_sm = 0;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 256, 0);
-            w.grid_ctas = std::min(GG_MAX_CTAS, sms * std::min(per_sm, 1));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 32 * GG_WARPS, 0);
+            w.grid_ctas = std::min({GG_MAX_CTAS, g_grid_ctas_limit.load(), sms * std::min(per_sm, 1)});
         }
     }
     {
@@ -3189,8 +3195,10 @@ uint64_t refine_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const Unit
             float2 *a32 = mw.a32;
             cx *vb = mw.v, *wb = mw.w;
             const int32_t *perm = mw.g_perm;
-            const cx *inv = mw.g_inv;
-            {
+            // a block's rows are dealt one to a warp (gg_block_solve): with
+            // fewer warps than rows, substitution in 32-row blocks
+            const cx *inv = GG_WARPS * mw.grid_ctas >= GI ? mw.g_inv : nullptr;
+            if (inv) {
                 const int sk = mw.grid_s[k];
                 set_smem_limit_once(k_gi_double, (int)(sizeof(cx) * GI / 2 * 32));
                 k_gi_base<<<(sk + 31) / 32, 64, 0, st>>>(d_solves, mw.mu, ui, mw.a32, status, mw.g_inv);
@@ -3205,7 +3213,7 @@ uint64_t refine_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const Unit
                             (void *)&perm, (void *)&inv, (void *)&mw.g_part, (void *)&mw.g_y, (void *)&mw.g_y2,
                             (void *)&mw.g_red, (void *)&gs};
             if (mw.grid_ctas <= 0 ||
-                launch_cooperative((const void *)k_gmres_grid, dim3(mw.grid_ctas), dim3(256), args, 0, st) !=
+                launch_cooperative((const void *)k_gmres_grid, dim3(mw.grid_ctas), dim3(32 * GG_WARPS), args, 0, st) !=
                     cudaSuccess) {
                 (void)cudaGetLastError();  // not co-resident: refine this solve in one CTA
                 k_gmres_ir<3><<<ns, 256, smem, st>>>(d_solves, d_ants, mw.mu, ibuf, crows, z, rhs, cosv, mw.a32, piv, x,
@@ -3542,6 +3550,11 @@ extern "C" int fnec_test_fill_rsqrt(const double *x, uint64_t n, double *out) {
     if (e == cudaSuccess) e = cudaMemcpy(out, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost);
     cudaFree(d);
     return e == cudaSuccess ? FNEC_OK : FNEC_ERR_CUDA;
+}
+
+extern "C" int fnec_test_limit_refinement_ctas(int32_t n) {
+    fnec::g_grid_ctas_limit = n > 0 ? n : fnec::GG_MAX_CTAS;
+    return FNEC_OK;
 }
 
 extern "C" int fnec_test_fill_sincospi(const double *x, uint64_t n, double *sin_out, double *cos_out) {

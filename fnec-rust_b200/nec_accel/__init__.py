@@ -197,6 +197,7 @@ SIGNATURES = {
     "fnec_batch_set_sources": (ctypes.c_int, [_P, _U32, _P, _U32]),
     "fnec_batch_resolve": (ctypes.c_int, [_P]),
     "fnec_test_fail_device_allocation": (ctypes.c_int, [_I32]),
+    "fnec_test_limit_refinement_ctas": (ctypes.c_int, [_I32]),
     "fnec_test_fill_sincospi": (ctypes.c_int, [_P, _U64, _P, _P]),
     "fnec_test_fill_rsqrt": (ctypes.c_int, [_P, _U64, _P]),
     "fnec_host_cache_release": (ctypes.c_int, [_P]),
@@ -607,6 +608,14 @@ def test_fail_device_allocation(after: int):
     rc = lib().fnec_test_fail_device_allocation(int(after))
     if rc != OK:
         raise AccelError(rc, "test_fail_device_allocation")
+
+
+def test_limit_refinement_ctas(n: int):
+    """Test hook: batches planned from now on refine grid-wide with at most
+    n CTAs, as on a partition of n SMs; 0: no limit."""
+    rc = lib().fnec_test_limit_refinement_ctas(int(n))
+    if rc != OK:
+        raise AccelError(rc, "test_limit_refinement_ctas")
 
 
 def host_cache_release() -> int:

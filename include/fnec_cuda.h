@@ -549,6 +549,9 @@ int fnec_selftest_tf32x3_gemm(int32_t device, uint64_t m, uint64_t n, uint64_t k
 int fnec_selftest_wait_timeout(int32_t device, int32_t which, uint64_t wait_ns, int32_t *unit_status,
                                double *elapsed_ms);
 int fnec_test_fail_device_allocation(int32_t after);
+/* fnec_test_limit_refinement_ctas(n): batches planned from now on refine
+ * grid-wide with at most n CTAs, as on a partition of n SMs; 0: no limit. */
+int fnec_test_limit_refinement_ctas(int32_t n);
 /* The mixed form's fill evaluates its samples' phase with its own
  * sin(pi x), cos(pi x) (quadrant reduction, Taylor series; the same source
  * is compiled for the host): fnec_test_fill_sincospi runs it on the host

@@ -64,3 +64,23 @@ def test_server_takes_a_large_request_whose_own_scratch_misses_the_budget(acc):
         assert status[0] == 0
         x0, x1 = np.ravel(ref.currents[0]), np.ravel(currents)
         assert np.linalg.norm(x1 - x0) <= 1e-7 * np.linalg.norm(x0)
+
+
+@pytest.mark.parametrize("ctas", [12, 31, 32])
+def test_refinement_on_few_sms(acc, ctas):
+    """A partition of fewer than 32 SMs has fewer warps than a diagonal block
+    has rows (8 a CTA, 256): the refinement still converges to the plain form
+    (its gates), as it does with 32."""
+    w, s, f = bench.mesh_workload(16)
+    ant = acc.Antenna(acc.wires_array(w), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    x0 = acc.HallenBatch([ant]).solve().currents[0]
+    acc.test_limit_refinement_ctas(ctas)
+    try:
+        b = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+    finally:
+        acc.test_limit_refinement_ctas(0)
+    assert b.units[0]["s"] >= 1536
+    r = b.solve()
+    assert r.status[0] == 0
+    assert np.linalg.norm(r.currents[0] - x0) <= 1e-7 * np.linalg.norm(x0)
+    assert b.refinement_stats()[0][0] < 24
