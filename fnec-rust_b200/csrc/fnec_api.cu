@@ -1849,6 +1849,7 @@ static int run_pipeline(fnec_batch *b) {
     };
     const char *failed = nullptr;  // the first phase whose launches failed
     std::string detail;
+    cudaError_t launch_error = cudaSuccess;
     auto check = [&](const char *phase) {
         if (!failed && cudaPeekAtLastError() != cudaSuccess) failed = phase;
     };
@@ -1887,6 +1888,7 @@ static int run_pipeline(fnec_batch *b) {
                        b->z_given.empty(), b->max_w, b->grid, mm, st, b->d_stamps, (int)b->stamps.size());
         if (!failed && mm.failed_phase) failed = mm.failed_phase;
         if (mm.detail[0]) detail = mm.detail;
+        launch_error = mm.error;
     } else {
         if (b->z_given.empty()) {
             launch_fill_exact(b->d_units, b->d_ants, b->d_segs, b->d_fill_tiles, (int)b->n_fill,
@@ -1992,6 +1994,7 @@ static int run_pipeline(fnec_batch *b) {
     check("far field");
     b->launches = L;
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_error;
     if (e != cudaSuccess)
         return fail(ctx, FNEC_ERR_CUDA, std::string(failed ? failed : "run") + ": " + cudaGetErrorString(e) +
                                             (detail.empty() ? "" : " [" + detail + "]"));

@@ -3236,7 +3236,11 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
     static const char *const phase_name[4] = {"fill", "gram", "factor", "refinement"};
     auto mark = [&](int k) {
         if (!marks.failed_phase && cudaPeekAtLastError() != cudaSuccess) marks.failed_phase = phase_name[k];
+        if (!marks.failed_phase && marks.error != cudaSuccess) marks.failed_phase = phase_name[k];
         if (marks.ev) cudaEventRecord(marks.ev[k], st);
+    };
+    auto launched = [&](cudaError_t e) {
+        if (marks.error == cudaSuccess) marks.error = e;
     };
     // the fill writes the Gram's tf32 operand stacks itself when the Gram
     // runs on the tensor cores and no stamp changes Z after the fill
@@ -3253,8 +3257,9 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
     }
     mark(0);
     if (mw.tc && mw.use_tc) {
-        tc_gram_run(*mw.tc, d_units, static_cast<const TcGramUnit *>(mw.tc_gu), static_cast<const TcTile *>(mw.tc_tiles),
-                    mw.smu, z, mw.tc_hi, mw.tc_lo, mw.a32, status, mw.tc_max_n, st, !fused_split, !mw.pivoting);
+        launched(tc_gram_run(*mw.tc, d_units, static_cast<const TcGramUnit *>(mw.tc_gu),
+                             static_cast<const TcTile *>(mw.tc_tiles), mw.smu, z, mw.tc_hi, mw.tc_lo, mw.a32, status,
+                             mw.tc_max_n, st, !fused_split, !mw.pivoting));
         ++L;
     } else if (n_gram > 0) {
         k_gram32_zz<<<n_gram, 256, 0, st>>>(d_units, mw.smu, gram_tiles, z, mw.a32);
@@ -3374,8 +3379,8 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
             }
         }
         if (mw.wide->active(C0 / WIDE) > 0) {
-            tc_trail_run(*mw.wide, C0 / WIDE, n_wide, static_cast<const TcTrailUnit *>(mw.d_wide), d_units, mw.smu,
-                         mw.a32, mw.wd_hi, mw.wd_lo, status, st, true);
+            launched(tc_trail_run(*mw.wide, C0 / WIDE, n_wide, static_cast<const TcTrailUnit *>(mw.d_wide), d_units,
+                                  mw.smu, mw.a32, mw.wd_hi, mw.wd_lo, status, st, true));
             L += 3;
         }
     }
@@ -3400,8 +3405,8 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
             ++L;
         }
         if (k_tc > 0) {
-            tc_trail_run(*mw.trail, c0 / MNB, k_tc, static_cast<const TcTrailUnit *>(mw.d_trail), d_units, mw.smu, mw.a32,
-                         mw.tr_hi, mw.tr_lo, status, fs, true);
+            launched(tc_trail_run(*mw.trail, c0 / MNB, k_tc, static_cast<const TcTrailUnit *>(mw.d_trail), d_units,
+                                  mw.smu, mw.a32, mw.tr_hi, mw.tr_lo, status, fs, true));
             L += 3;
         }
     }
@@ -3490,8 +3495,8 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
             ++L;
         }
         if (k_tc > 0) {
-            tc_trail_run(*mw.trail, c0 / MNB, k_tc, static_cast<const TcTrailUnit *>(mw.d_trail), d_units, mw.smu, mw.a32,
-                         mw.tr_hi, mw.tr_lo, status, fs);
+            launched(tc_trail_run(*mw.trail, c0 / MNB, k_tc, static_cast<const TcTrailUnit *>(mw.d_trail), d_units,
+                                  mw.smu, mw.a32, mw.tr_hi, mw.tr_lo, status, fs));
             L += 3;
         }
     }

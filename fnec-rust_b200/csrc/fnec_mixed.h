@@ -105,6 +105,7 @@ struct MixedMarks {
     cudaEvent_t *ev;
     const char *failed_phase = nullptr;  // set by run_mixed: the first phase whose launches failed
     char detail[160] = {0};               // the failed launch's shape, when known
+    cudaError_t error = cudaSuccess;      // of a launch whose own check has cleared it
 };
 
 bool mixed_available();

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <mutex>
 
@@ -698,6 +699,17 @@ bool make_map(CUtensorMap *m, const float *base, int64_t rows, int box_rows = BM
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Test hook (fnec_test_fail_tensor_launch): the n-th tensor-core launch of a
+// batch from now on is refused as if the device had no room for it (once).
+std::atomic<int> g_fail_launch_after{-1};
+bool take_injected_launch_failure() {
+    int v = g_fail_launch_after.load();
+    while (v >= 0) {
+        if (g_fail_launch_after.compare_exchange_weak(v, v - 1)) return v == 0;
+    }
+    return false;
+}
+
 size_t tc_smem_bytes() { return (size_t)STAGES * STAGE_BYTES + 1024; }
 
 template <int EPI>
@@ -806,6 +818,7 @@ cudaError_t tc_trail_run(const TcTrailPlan &p, int step, int count, const TcTrai
                          bool lower, bool persistent) {
     const int na = std::min(count, p.active(step));
     if (na <= 0) return cudaSuccess;
+    if (take_injected_launch_failure()) return cudaErrorLaunchOutOfResources;
     const TcTrailUnit *tl = d_trail + p.u_off[step];
     const int c0 = 32 * p.parts * step;
     const unsigned parts = (unsigned)p.parts;
@@ -860,6 +873,7 @@ cudaError_t tc_gram_run(const TcGramPlan &p, const UnitDesc *d_units, const TcGr
                         const MixedUnit *d_mus, const cx *z, float *hi, float *lo, float2 *a32, int32_t *status,
                         int max_n, cudaStream_t st, bool split, bool lower_only) {
     if (p.units.empty()) return cudaSuccess;
+    if (take_injected_launch_failure()) return cudaErrorLaunchOutOfResources;
     if (split) {  // else the fill has written the stacks
         int max_kb = (max_n + 31) / 32, max_cb = (max_n + 15) / 16;
         dim3 g(max_cb, max_kb, (unsigned)p.units.size());
@@ -975,6 +989,11 @@ static int tc_selftest(int32_t device, uint64_t m, uint64_t n, uint64_t k, const
     cudaFree(dt);
     cudaFree(dst);
     return rc;
+}
+
+extern "C" int fnec_test_fail_tensor_launch(int32_t after) {
+    g_fail_launch_after = after < 0 ? -1 : after;
+    return FNEC_OK;
 }
 
 extern "C" int fnec_selftest_tf32x3_gemm(int32_t device, uint64_t m, uint64_t n, uint64_t k, const float *a,

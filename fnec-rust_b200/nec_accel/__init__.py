@@ -197,6 +197,7 @@ SIGNATURES = {
     "fnec_batch_set_sources": (ctypes.c_int, [_P, _U32, _P, _U32]),
     "fnec_batch_resolve": (ctypes.c_int, [_P]),
     "fnec_test_fail_device_allocation": (ctypes.c_int, [_I32]),
+    "fnec_test_fail_tensor_launch": (ctypes.c_int, [_I32]),
     "fnec_test_limit_refinement_ctas": (ctypes.c_int, [_I32]),
     "fnec_test_fill_sincospi": (ctypes.c_int, [_P, _U64, _P, _P]),
     "fnec_test_fill_rsqrt": (ctypes.c_int, [_P, _U64, _P]),
@@ -608,6 +609,14 @@ def test_fail_device_allocation(after: int):
     rc = lib().fnec_test_fail_device_allocation(int(after))
     if rc != OK:
         raise AccelError(rc, "test_fail_device_allocation")
+
+
+def test_fail_tensor_launch(after: int):
+    """Test hook: the after-th tensor-core launch of a batch from now on is
+    refused (once); -1 disarms."""
+    rc = lib().fnec_test_fail_tensor_launch(int(after))
+    if rc != OK:
+        raise AccelError(rc, "test_fail_tensor_launch")
 
 
 def test_limit_refinement_ctas(n: int):

@@ -549,6 +549,9 @@ int fnec_selftest_tf32x3_gemm(int32_t device, uint64_t m, uint64_t n, uint64_t k
 int fnec_selftest_wait_timeout(int32_t device, int32_t which, uint64_t wait_ns, int32_t *unit_status,
                                double *elapsed_ms);
 int fnec_test_fail_device_allocation(int32_t after);
+/* fnec_test_fail_tensor_launch(n): the n-th tensor-core launch of a batch
+ * (Gram, trailing updates) from now on is refused (once); -1 disarms. */
+int fnec_test_fail_tensor_launch(int32_t after);
 /* fnec_test_limit_refinement_ctas(n): batches planned from now on refine
  * grid-wide with at most n CTAs, as on a partition of n SMs; 0: no limit. */
 int fnec_test_limit_refinement_ctas(int32_t n);

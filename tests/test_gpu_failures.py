@@ -162,3 +162,29 @@ def test_non_finite_geometry_is_refused_for_that_antenna_only(acc):
             assert np.array_equal(np.asarray(cur).reshape(-1).view(np.uint64),
                                   alone[r.tag].reshape(-1).view(np.uint64))
             r.release()
+
+
+@pytest.mark.parametrize("after", [0, 1, 20])
+def test_refused_tensor_launch_is_reported(acc, after):
+    """The Gram's launch (0), or one of the 128-column trailing updates of a
+    system of S = 3,360, refused by the host: the run reports the error (a
+    factor that misses an update is not handed on as solved), and the same
+    batch solves when it is run again."""
+    import bench
+
+    w, s, f = bench.mesh_workload(24)
+    ant = acc.Antenna(acc.wires_array(w[:1120]), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    b = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+    assert b.units[0]["s"] == 3360
+    acc.test_fail_tensor_launch(after)
+    try:
+        with pytest.raises(acc.AccelError) as ei:
+            b.solve()
+        assert ei.value.code == acc.ERR_CUDA
+    finally:
+        acc.test_fail_tensor_launch(-1)
+    r = b.solve()
+    x0 = acc.HallenBatch([ant]).solve().currents[0]
+    assert r.status[0] == 0
+    assert np.linalg.norm(r.currents[0] - x0) <= 1e-7 * np.linalg.norm(x0)
+    b.close()
