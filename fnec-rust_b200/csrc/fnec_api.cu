@@ -726,6 +726,7 @@ struct fnec_batch {
     bool pooled = false;
     bool dev_pool = true;
     bool allow_grid = true;
+    bool large_scratch = true;
     unsigned char *stage = nullptr;  // page-locked staging of uploads (pooled batches)
     size_t stage_cap = 0, stage_used = 0;
     double alloc_ms = 0;  // host time spent allocating (device pool, pinned arenas, mixed work)
@@ -970,7 +971,8 @@ static void apply_schedule(fnec_batch *b, const fnec_schedule &s);
 struct BatchPlace {
     cudaStream_t st = nullptr;  // null: the context's stream
     bool pooled = false;
-    bool allow_grid = true;
+    bool allow_grid = true;     // cooperative launches
+    bool large_scratch = true;  // the large systems' optional scratch (alloc_mixed)
     PinnedArena *in = nullptr, *out = nullptr;  // pooled only
     PinnedArena *aux = nullptr;                 // pooled only: staging of the other uploads
 };
@@ -989,6 +991,7 @@ static int build_batch(fnec_ctx *ctx, std::vector<HostAnt> &hs, int precision, f
     b->st = place.st ? place.st : ctx->stream;
     b->pooled = place.pooled;
     b->allow_grid = place.allow_grid;
+    b->large_scratch = place.large_scratch;
     if (place.aux) {
         b->stage = place.aux->p;
         b->stage_cap = place.aux->cap;
@@ -1415,7 +1418,8 @@ static int build_batch(fnec_ctx *ctx, std::vector<HostAnt> &hs, int precision, f
     if (e == cudaSuccess && precision == FNEC_PRECISION_MIXED) {
         const auto tm = std::chrono::steady_clock::now();
         e = alloc_mixed(b->mixed, b->units, b->solves, b->ants, b->max_s,
-                        DevAlloc{b->st, b->dev_pool, b->stage, b->stage_cap, &b->stage_used}, b->allow_grid);
+                        DevAlloc{b->st, b->dev_pool, b->stage, b->stage_cap, &b->stage_used, take_injected_alloc_failure},
+                        b->allow_grid, b->large_scratch);
         b->t_mixed += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tm).count();
     }
     b->alloc_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - ta0).count();
@@ -3128,7 +3132,7 @@ struct ServerReq {
     fnec_request_out out{};
     bool copy_out = false;
     int64_t bytes = 0;
-    bool large = false;  // bytes holds the large systems' own scratch
+    bool large = false;  // bytes holds the large systems' optional scratch
     uint32_t n_solves = 0, n = 0, s = 0, n_points = 0, n_feed_rows = 0;
     Clock::time_point t_submit, t_done;
     int32_t state = FNEC_REQ_QUEUED;
@@ -3148,8 +3152,8 @@ struct Lane {
 
 // Upper bound of the device bytes one request's batch needs (Z, the
 // factor, solution and work vectors, Gram operand stacks, pattern buffers).
-// large: with the scratch that only a batch planned with allow_grid takes
-// (the wide factor steps', the grid-wide refinement's block inverses).
+// large: with the large systems' optional scratch (the wide factor steps',
+// the grid-wide refinement's block inverses).
 int64_t request_bytes(const HostAnt &h, int precision, bool large = true) {
     const int64_t n = (int64_t)h.segs.size(), w = h.cols(), s = n + w;
     const int64_t f = (int64_t)h.freqs.size(), r = (int64_t)std::max<size_t>(h.rhs_srcs.size(), 1);
@@ -3337,7 +3341,7 @@ void lane_worker(fnec_server *S, Lane *L) {
         }
         std::vector<HostAnt> hs;
         hs.reserve(take.size());
-        bool large = S->lanes.size() == 1;  // cooperative kernels need the whole device
+        bool large = true;
         for (ServerReq *r : take) {
             hs.push_back(r->host);
             large = large && r->large;
@@ -3345,7 +3349,8 @@ void lane_worker(fnec_server *S, Lane *L) {
         BatchPlace place;
         place.st = L->st;
         place.pooled = true;
-        place.allow_grid = large;
+        place.allow_grid = S->lanes.size() == 1;  // cooperative kernels need the whole device
+        place.large_scratch = large;
         place.in = &L->in;
         place.out = &slab->mem;
         place.aux = &L->aux;
@@ -3561,8 +3566,8 @@ int fnec_server_submit(fnec_server *S, const fnec_antenna *req, const fnec_reque
     for (auto &v : h.rhs_feeds) fr += (uint32_t)v.size();
     r->n_feed_rows = fr * (uint32_t)h.freqs.size();
     r->status.assign(r->n_solves, 0);
-    // a request whose large systems' scratch would not fit the budget, or
-    // whose lane could not use it, is planned and counted without it
+    // a request whose large systems' optional scratch would not fit the
+    // budget, or of a server of several lanes, is planned and counted without it
     const int64_t full = request_bytes(h, S->cfg.precision);
     r->large = S->lanes.size() == 1 && full <= (int64_t)S->cfg.hbm_budget_bytes;
     r->bytes = r->large ? full : request_bytes(h, S->cfg.precision, false);

@@ -38,7 +38,9 @@ struct DevAlloc {
     unsigned char *stage = nullptr;
     size_t stage_cap = 0;
     size_t *stage_used = nullptr;
+    bool (*fail)() = nullptr;  // test hook: this allocation fails
     cudaError_t alloc(void **p, size_t bytes) const {
+        if (fail && fail()) return cudaErrorMemoryAllocation;
         return pooled ? cudaMallocAsync(p, bytes, st) : cudaMalloc(p, bytes);
     }
     cudaError_t upload(void *dst, const void *src, size_t bytes) const {

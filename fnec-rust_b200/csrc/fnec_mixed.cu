@@ -2771,7 +2771,8 @@ bool mixed_available() { return true; }
 static std::atomic<int> g_grid_ctas_limit{GG_MAX_CTAS};
 
 cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, const std::vector<UnitDesc> &solves,
-                        const std::vector<AntDesc> &ants, int max_s, const DevAlloc &dev, bool allow_grid) {
+                        const std::vector<AntDesc> &ants, int max_s, const DevAlloc &dev, bool allow_grid,
+                        bool large_scratch) {
     std::vector<int64_t> a32_of(systems.size()), binv_of(systems.size());
     int64_t a32 = 0, v = 0, wk = 0, binv = 0;
     for (size_t i = 0; i < systems.size(); ++i) {
@@ -2893,10 +2894,9 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             partmax = std::max<int64_t>(partmax, (int64_t)((u.n + GG_RC - 1) / GG_RC) * u.n);
         }
         size_t b_perm = sizeof(int32_t) * (size_t)smax, b_part = sizeof(cx) * (size_t)partmax,
-               b_y = sizeof(cx) * (size_t)smax, b_inv = sizeof(cx) * 2 * GI * GI * (size_t)((smax + GI - 1) / GI),
-               b_red = sizeof(cx) * 2 * GG_MAX_CTAS * (GM + 1),
+               b_y = sizeof(cx) * (size_t)smax, b_red = sizeof(cx) * 2 * GG_MAX_CTAS * (GM + 1),
                b_sync = sizeof(GridSync) * w.grid_solves.size();
-        size_t gt = al(b_perm) + al(b_part) + 2 * al(b_y) + al(b_inv) + al(b_red) + al(b_sync);
+        size_t gt = al(b_perm) + al(b_part) + al(b_y) + al(b_red) + al(b_sync);
         e = dev.alloc(&w.grid_base, gt);
         if (e == cudaErrorMemoryAllocation) {  // no room for it: these solves refine in one CTA each
             (void)cudaGetLastError();
@@ -2914,19 +2914,31 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             q += al(b_part);
             w.g_y = (cx *)q;
             q += al(b_y);
-            w.g_y2 = (cx *)q;
-            q += al(b_y);
-            w.g_inv = (cx *)q;
-            q += al(b_inv);
             w.g_red = (cx *)q;
             q += al(b_red);
             w.g_sync = q;
             w.bytes += gt;
-            int dev = 0, sms = 0, per_sm = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            int device = 0, sms = 0, per_sm = 0;
+            cudaGetDevice(&device);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 32 * GG_WARPS, 0);
             w.grid_ctas = std::min({GG_MAX_CTAS, g_grid_ctas_limit.load(), sms * std::min(per_sm, 1)});
+            // the block inverses, for a grid of at least a warp per row of a
+            // block (gg_block_solve deals them so)
+            const size_t b_inv = sizeof(cx) * 2 * GI * GI * (size_t)((smax + GI - 1) / GI);
+            if (large_scratch && GG_WARPS * w.grid_ctas >= GI) {
+                e = dev.alloc(&w.inv_base, al(b_y) + al(b_inv));
+                if (e == cudaSuccess) {
+                    w.g_y2 = (cx *)w.inv_base;
+                    w.g_inv = (cx *)((unsigned char *)w.inv_base + al(b_y));
+                    w.bytes += al(b_y) + al(b_inv);
+                } else if (e == cudaErrorMemoryAllocation) {  // no room for them: substitution in 32-row blocks
+                    (void)cudaGetLastError();
+                    w.inv_base = nullptr;
+                } else {
+                    return e;
+                }
+            }
         }
     }
     {
@@ -3035,7 +3047,7 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
         }
         int n_wide = 0;
         while (n_wide < (int)sd.size() && sd[n_wide] >= WIDE_MIN_S) ++n_wide;
-        if (allow_grid && n_wide > 0 && n_wide <= TC_WIDE_MAX_UNITS && w.tc && tc_wide_ready()) {
+        if (large_scratch && n_wide > 0 && n_wide <= TC_WIDE_MAX_UNITS && w.tc && tc_wide_ready()) {
             TcTrailPlan *p = new TcTrailPlan();
             tc_trail_plan(sd, ord, n_wide, 1, WIDE / MNB, *p);
             size_t b_st = sizeof(float) * 32 * (size_t)p->rows, b_u = sizeof(TcTrailUnit) * (p->units.size() + 1);
@@ -3095,6 +3107,7 @@ void free_mixed(MixedWork &w, const DevAlloc &dev) {
     w.fmade = false;
     dev.release(w.base);
     dev.release(w.grid_base);
+    dev.release(w.inv_base);
     dev.release(w.tc_base);
     dev.release(w.c_base);
     dev.release(w.trail_base);
@@ -3110,6 +3123,8 @@ void free_mixed(MixedWork &w, const DevAlloc &dev) {
     w.c_base = nullptr;
     w.c_scratch = nullptr;
     w.grid_base = nullptr;
+    w.inv_base = nullptr;
+    w.g_inv = w.g_y2 = nullptr;
     w.tc_base = nullptr;
     delete w.tc;
     w.tc = nullptr;
@@ -3195,9 +3210,7 @@ uint64_t refine_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const Unit
             float2 *a32 = mw.a32;
             cx *vb = mw.v, *wb = mw.w;
             const int32_t *perm = mw.g_perm;
-            // a block's rows are dealt one to a warp (gg_block_solve): with
-            // fewer warps than rows, substitution in 32-row blocks
-            const cx *inv = GG_WARPS * mw.grid_ctas >= GI ? mw.g_inv : nullptr;
+            const cx *inv = mw.g_inv;
             if (inv) {
                 const int sk = mw.grid_s[k];
                 set_smem_limit_once(k_gi_double, (int)(sizeof(cx) * GI / 2 * 32));

@@ -53,8 +53,10 @@ struct MixedWork {
     void *grid_base = nullptr;     // scratch shared by those launches
     int32_t *g_perm = nullptr;
     cx *g_part = nullptr;
-    cx *g_y = nullptr, *g_y2 = nullptr;  // substitution vectors
-    cx *g_inv = nullptr;                 // inverses of the factor's 256-row diagonal blocks
+    cx *g_y = nullptr;             // substitution vector
+    void *inv_base = nullptr;      // optional: inverses of the factor's 256-row diagonal blocks and the
+    cx *g_inv = nullptr;           // second vector they take (null: substitution in 32-row blocks)
+    cx *g_y2 = nullptr;
     cx *g_red = nullptr;
     void *g_sync = nullptr;
     int grid_ctas = 0;
@@ -110,11 +112,12 @@ struct MixedMarks {
 
 bool mixed_available();
 // systems: one per factorisation; solves: one per right-hand side.
-// allow_grid: large solves may take the grid-wide (cooperative) GMRES and large
-// Hermitian systems the wide factor steps, each with its own scratch (without
-// room for it they take the paths of smaller systems)
+// allow_grid: large solves may take the grid-wide (cooperative) GMRES.
+// large_scratch: they may also take its block inverses, and large Hermitian
+// systems the wide factor steps, each where the device has room for its scratch
 cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, const std::vector<UnitDesc> &solves,
-                        const std::vector<AntDesc> &ants, int max_s, const DevAlloc &dev, bool allow_grid);
+                        const std::vector<AntDesc> &ants, int max_s, const DevAlloc &dev, bool allow_grid,
+                        bool large_scratch);
 void free_mixed(MixedWork &w, const DevAlloc &dev);
 // Enqueue fill + Gram + factor + refinement for all units; returns the
 // number of kernel launches issued.

@@ -84,3 +84,53 @@ def test_refinement_on_few_sms(acc, ctas):
     assert r.status[0] == 0
     assert np.linalg.norm(r.currents[0] - x0) <= 1e-7 * np.linalg.norm(x0)
     assert b.refinement_stats()[0][0] < 24
+
+
+def test_no_room_for_the_inverses_keeps_the_grid_refinement(acc):
+    """A batch whose allocation of the block inverses fails (the last one of
+    its planning; injected) still refines grid-wide, in 32-row blocks: it
+    runs the launches of a full one but for the four that form the inverses."""
+    w, s, f = bench.mesh_workload(16)
+    ant = acc.Antenna(acc.wires_array(w), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    full = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+    ref = full.solve()
+    seen = set()
+    for after in range(60):
+        acc.test_fail_device_allocation(after)
+        try:
+            b = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+        except acc.AccelError as e:
+            assert e.code == acc.ERR_OUT_OF_MEMORY
+            continue
+        finally:
+            acc.test_fail_device_allocation(-1)
+        if b.info.device_bytes == full.info.device_bytes:
+            break  # nothing failed: past the last allocation
+        r = b.solve()
+        assert r.status[0] == 0
+        assert np.linalg.norm(r.currents[0] - ref.currents[0]) <= 1e-7 * np.linalg.norm(ref.currents[0])
+        seen.add(full.kernel_launches - b.kernel_launches)
+        b.close()
+    assert 4 in seen
+
+
+def _serve(acc, ants, **kw):
+    with acc.Server(acc.PRECISION_MIXED, lanes=1, **kw) as srv:
+        reqs = [srv.submit(a, copy_out=True) for a in ants]
+        for r in reqs:
+            srv.wait(r)
+        return [r.result() for r in reqs], srv.stats()
+
+
+def test_request_without_the_optional_scratch_still_refines_grid_wide(acc):
+    """The budget of the test above, seen in the launches: the request runs
+    all of a full one's but the four that form the block inverses."""
+    w, s, f = bench.mesh_workload(16)
+    ant = acc.Antenna(acc.wires_array(w), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    with acc.Server(acc.PRECISION_MIXED, lanes=1, hbm_budget_bytes=1 << 30) as srv:
+        need = srv.shape(ant).device_bytes
+    (full,), s0 = _serve(acc, [ant], hbm_budget_bytes=1 << 30)
+    (lean,), s1 = _serve(acc, [ant], hbm_budget_bytes=need - (4 << 20))
+    assert full[3][0] == 0 and lean[3][0] == 0
+    assert s0["kernel_launches"] - s1["kernel_launches"] == 4
+    assert np.linalg.norm(lean[0][0] - full[0][0]) <= 1e-7 * np.linalg.norm(full[0][0])
