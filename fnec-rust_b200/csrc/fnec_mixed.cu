@@ -2886,61 +2886,6 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
         w.grid_solves.clear();
         w.grid_s.clear();
     }
-    if (!w.grid_solves.empty()) {
-        int64_t smax = 0, partmax = 0;
-        for (int i : w.grid_solves) {
-            const UnitDesc &u = solves[i];
-            smax = std::max<int64_t>(smax, u.s);
-            partmax = std::max<int64_t>(partmax, (int64_t)((u.n + GG_RC - 1) / GG_RC) * u.n);
-        }
-        size_t b_perm = sizeof(int32_t) * (size_t)smax, b_part = sizeof(cx) * (size_t)partmax,
-               b_y = sizeof(cx) * (size_t)smax, b_red = sizeof(cx) * 2 * GG_MAX_CTAS * (GM + 1),
-               b_sync = sizeof(GridSync) * w.grid_solves.size();
-        size_t gt = al(b_perm) + al(b_part) + al(b_y) + al(b_red) + al(b_sync);
-        e = dev.alloc(&w.grid_base, gt);
-        if (e == cudaErrorMemoryAllocation) {  // no room for it: these solves refine in one CTA each
-            (void)cudaGetLastError();
-            w.grid_base = nullptr;
-            w.grid_solves.clear();
-            w.grid_s.clear();
-            e = cudaSuccess;
-        }
-        if (e != cudaSuccess) return e;
-        if (w.grid_base) {
-            unsigned char *q = (unsigned char *)w.grid_base;
-            w.g_perm = (int32_t *)q;
-            q += al(b_perm);
-            w.g_part = (cx *)q;
-            q += al(b_part);
-            w.g_y = (cx *)q;
-            q += al(b_y);
-            w.g_red = (cx *)q;
-            q += al(b_red);
-            w.g_sync = q;
-            w.bytes += gt;
-            int device = 0, sms = 0, per_sm = 0;
-            cudaGetDevice(&device);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 32 * GG_WARPS, 0);
-            w.grid_ctas = std::min({GG_MAX_CTAS, g_grid_ctas_limit.load(), sms * std::min(per_sm, 1)});
-            // the block inverses, for a grid of at least a warp per row of a
-            // block (gg_block_solve deals them so)
-            const size_t b_inv = sizeof(cx) * 2 * GI * GI * (size_t)((smax + GI - 1) / GI);
-            if (large_scratch && GG_WARPS * w.grid_ctas >= GI) {
-                e = dev.alloc(&w.inv_base, al(b_y) + al(b_inv));
-                if (e == cudaSuccess) {
-                    w.g_y2 = (cx *)w.inv_base;
-                    w.g_inv = (cx *)((unsigned char *)w.inv_base + al(b_y));
-                    w.bytes += al(b_y) + al(b_inv);
-                } else if (e == cudaErrorMemoryAllocation) {  // no room for them: substitution in 32-row blocks
-                    (void)cudaGetLastError();
-                    w.inv_base = nullptr;
-                } else {
-                    return e;
-                }
-            }
-        }
-    }
     {
         // cluster GMRES when one CTA per solve cannot fill the GPU
         int device = 0, sms = 0;
@@ -3010,14 +2955,14 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             delete p;
         }
     }
+    std::vector<int32_t> ord(systems.size());  // systems by decreasing S
+    for (size_t i = 0; i < ord.size(); ++i) ord[i] = (int32_t)i;
+    std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return systems[x].s > systems[y].s; });
+    std::vector<int> sd(ord.size());
+    for (size_t i = 0; i < ord.size(); ++i) sd[i] = systems[ord[i]].s;
     {
         // tensor-core trailing updates: units whose first trailing block has
         // at least TC_TRAIL_MIN_M rows, while it still does
-        std::vector<int32_t> ord(systems.size());
-        for (size_t i = 0; i < ord.size(); ++i) ord[i] = (int32_t)i;
-        std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return systems[x].s > systems[y].s; });
-        std::vector<int> sd(ord.size());
-        for (size_t i = 0; i < ord.size(); ++i) sd[i] = systems[ord[i]].s;
         int n_tc = 0;
         while (n_tc < (int)sd.size() && sd[n_tc] - 32 >= TC_TRAIL_MIN_M) ++n_tc;
         if (n_tc > 0 && w.tc) {
@@ -3045,6 +2990,49 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
             w.trail = p;
             w.trail_n = n_tc;
         }
+    }
+    // What follows a batch can do without: it is allocated last, so that it takes
+    // no room from what the batch needs.
+    if (!w.grid_solves.empty()) {
+        int64_t smax = 0, partmax = 0;
+        for (int i : w.grid_solves) {
+            const UnitDesc &u = solves[i];
+            smax = std::max<int64_t>(smax, u.s);
+            partmax = std::max<int64_t>(partmax, (int64_t)((u.n + GG_RC - 1) / GG_RC) * u.n);
+        }
+        size_t b_perm = sizeof(int32_t) * (size_t)smax, b_part = sizeof(cx) * (size_t)partmax,
+               b_y = sizeof(cx) * (size_t)smax, b_red = sizeof(cx) * 2 * GG_MAX_CTAS * (GM + 1),
+               b_sync = sizeof(GridSync) * w.grid_solves.size();
+        size_t gt = al(b_perm) + al(b_part) + al(b_y) + al(b_red) + al(b_sync);
+        e = dev.alloc(&w.grid_base, gt);
+        if (e == cudaErrorMemoryAllocation) {  // no room for it: these solves refine in one CTA each
+            (void)cudaGetLastError();
+            w.grid_base = nullptr;
+            w.grid_solves.clear();
+            w.grid_s.clear();
+            e = cudaSuccess;
+        }
+        if (e != cudaSuccess) return e;
+        if (w.grid_base) {
+            unsigned char *q = (unsigned char *)w.grid_base;
+            w.g_perm = (int32_t *)q;
+            q += al(b_perm);
+            w.g_part = (cx *)q;
+            q += al(b_part);
+            w.g_y = (cx *)q;
+            q += al(b_y);
+            w.g_red = (cx *)q;
+            q += al(b_red);
+            w.g_sync = q;
+            w.bytes += gt;
+            int device = 0, sms = 0, per_sm = 0;
+            cudaGetDevice(&device);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_grid, 32 * GG_WARPS, 0);
+            w.grid_ctas = std::min({GG_MAX_CTAS, g_grid_ctas_limit.load(), sms * std::min(per_sm, 1)});
+        }
+    }
+    {
         int n_wide = 0;
         while (n_wide < (int)sd.size() && sd[n_wide] >= WIDE_MIN_S) ++n_wide;
         if (large_scratch && n_wide > 0 && n_wide <= TC_WIDE_MAX_UNITS && w.tc && tc_wide_ready()) {
@@ -3080,6 +3068,23 @@ cudaError_t alloc_mixed(MixedWork &w, const std::vector<UnitDesc> &systems, cons
                 w.wide = p;
                 w.wide_n = n_wide;
             }
+        }
+    }
+    // the block inverses, for a grid of at least a warp per row of a block
+    // (gg_block_solve deals them so)
+    if (large_scratch && !w.grid_solves.empty() && GG_WARPS * w.grid_ctas >= GI) {
+        const int smax = *std::max_element(w.grid_s.begin(), w.grid_s.end());
+        const size_t b_y = sizeof(cx) * (size_t)smax, b_inv = sizeof(cx) * 2 * GI * GI * (size_t)((smax + GI - 1) / GI);
+        e = dev.alloc(&w.inv_base, al(b_y) + al(b_inv));
+        if (e == cudaSuccess) {
+            w.g_y2 = (cx *)w.inv_base;
+            w.g_inv = (cx *)((unsigned char *)w.inv_base + al(b_y));
+            w.bytes += al(b_y) + al(b_inv);
+        } else if (e == cudaErrorMemoryAllocation) {  // no room for them: substitution in 32-row blocks
+            (void)cudaGetLastError();
+            w.inv_base = nullptr;
+        } else {
+            return e;
         }
     }
     if (systems.size() >= 4 && !w.fmade) {  // concurrent factor groups

@@ -188,3 +188,35 @@ def test_refused_tensor_launch_is_reported(acc, after):
     assert r.status[0] == 0
     assert np.linalg.norm(r.currents[0] - x0) <= 1e-7 * np.linalg.norm(x0)
     b.close()
+
+
+def test_optional_scratch_is_allocated_last(acc):
+    """S = 3,360 takes every optional allocation (grid-wide refinement, its
+    block inverses, 128-column steps).  With the n-th allocation failing,
+    planning fails for each one the batch needs and succeeds for each one it
+    does not; the optional ones come last, so they never take the room of a
+    needed one."""
+    import bench
+
+    w, s, f = bench.mesh_workload(24)
+    ant = acc.Antenna(acc.wires_array(w[:1120]), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    whole = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+    planned = []
+    for after in range(80):
+        acc.test_fail_device_allocation(after)
+        try:
+            b = acc.HallenBatch([ant], precision=acc.PRECISION_MIXED)
+        except acc.AccelError as e:
+            assert e.code == acc.ERR_OUT_OF_MEMORY
+            planned.append(False)
+            continue
+        finally:
+            acc.test_fail_device_allocation(-1)
+        done = b.info.device_bytes == whole.info.device_bytes
+        b.close()
+        if done:
+            break
+        planned.append(True)
+    n = planned.index(True)
+    assert planned == [False] * n + [True] * 3
+    whole.close()
