@@ -3132,7 +3132,9 @@ struct ServerReq {
     fnec_request_out out{};
     bool copy_out = false;
     int64_t bytes = 0;
-    bool large = false;  // bytes holds the large systems' optional scratch
+    // the large systems' optional scratch: taken (bytes holds it), left out,
+    // or not asked for
+    enum { SCRATCH_NONE, SCRATCH_TAKEN, SCRATCH_LEFT_OUT } scratch = SCRATCH_NONE;
     uint32_t n_solves = 0, n = 0, s = 0, n_points = 0, n_feed_rows = 0;
     Clock::time_point t_submit, t_done;
     int32_t state = FNEC_REQ_QUEUED;
@@ -3233,12 +3235,19 @@ void slab_unref(fnec_server *S, Slab *sl) {  // S->mu held
 }
 
 // Takes the next batch (arrival order, within budget and max_batch); S->mu held.
+// A batch plans its optional scratch for all of its requests or for none, so
+// one that must leave it out does not share a batch with one that takes it.
 std::vector<ServerReq *> admit(fnec_server *S, int64_t &bytes) {
     std::vector<ServerReq *> take;
     bytes = 0;
+    int scratch = ServerReq::SCRATCH_NONE;
     while (!S->queue.empty() && take.size() < S->cfg.max_batch) {
         ServerReq *r = S->queue.front();
         if (S->in_flight + bytes + r->bytes > (int64_t)S->cfg.hbm_budget_bytes) break;
+        if (r->scratch != ServerReq::SCRATCH_NONE) {
+            if (scratch != ServerReq::SCRATCH_NONE && scratch != r->scratch) break;
+            scratch = r->scratch;
+        }
         bytes += r->bytes;
         take.push_back(r);
         S->queue.pop_front();
@@ -3344,7 +3353,7 @@ void lane_worker(fnec_server *S, Lane *L) {
         bool large = true;
         for (ServerReq *r : take) {
             hs.push_back(r->host);
-            large = large && r->large;
+            large = large && r->scratch != ServerReq::SCRATCH_LEFT_OUT;
         }
         BatchPlace place;
         place.st = L->st;
@@ -3569,8 +3578,10 @@ int fnec_server_submit(fnec_server *S, const fnec_antenna *req, const fnec_reque
     // a request whose large systems' optional scratch would not fit the
     // budget, or of a server of several lanes, is planned and counted without it
     const int64_t full = request_bytes(h, S->cfg.precision);
-    r->large = S->lanes.size() == 1 && full <= (int64_t)S->cfg.hbm_budget_bytes;
-    r->bytes = r->large ? full : request_bytes(h, S->cfg.precision, false);
+    const bool large = S->lanes.size() == 1 && full <= (int64_t)S->cfg.hbm_budget_bytes;
+    r->bytes = large ? full : request_bytes(h, S->cfg.precision, false);
+    if (r->bytes != full) r->scratch = ServerReq::SCRATCH_LEFT_OUT;
+    else if (full != request_bytes(h, S->cfg.precision, false)) r->scratch = ServerReq::SCRATCH_TAKEN;
     if (info) {
         info->n_segments = r->n;
         info->n_rhs = (uint32_t)std::max<size_t>(h.rhs_srcs.size(), 1);

@@ -134,3 +134,38 @@ def test_request_without_the_optional_scratch_still_refines_grid_wide(acc):
     assert full[3][0] == 0 and lean[3][0] == 0
     assert s0["kernel_launches"] - s1["kernel_launches"] == 4
     assert np.linalg.norm(lean[0][0] - full[0][0]) <= 1e-7 * np.linalg.norm(full[0][0])
+
+
+def test_request_without_the_optional_scratch_leaves_the_others_theirs(acc):
+    """S = 9,840, 120, 1,632 and 120, all queued before the only lane may take
+    one (results held in place fill its five slabs), on a budget with no room
+    for the first one's optional scratch but for its other needs beside all
+    of the others.  Two batches: one without the scratch, with the first
+    small request in it, and one with it."""
+    def ant(w, f):
+        return acc.Antenna(acc.wires_array(w), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+
+    w, s, f = bench.mesh_workload(40)
+    big, mid, small = ant(w, f), ant(w[:544], f), ant(w[:40], f)
+    with acc.Server(acc.PRECISION_MIXED, lanes=1, hbm_budget_bytes=8 << 30) as srv:
+        budget = srv.shape(big).device_bytes - (10 << 20)
+
+    def burst(ants):
+        with acc.Server(acc.PRECISION_MIXED, lanes=1, hbm_budget_bytes=budget) as srv:
+            held = [srv.wait(srv.submit(small)) for _ in range(5)]
+            srv.stats(reset=True)
+            reqs = [srv.submit(a, copy_out=True) for a in ants]
+            for r in held:
+                r.release()
+            for r in reqs:
+                srv.wait(r)
+            return reqs, srv.stats()
+
+    reqs, st = burst([big, small, mid, small])
+    first, s1 = burst([big, small])
+    second, s2 = burst([mid, small])
+    assert (st["batches"], s1["batches"], s2["batches"]) == (2, 1, 1)
+    assert st["kernel_launches"] == s1["kernel_launches"] + s2["kernel_launches"]
+    for a, b in zip(reqs, first + second):
+        assert a.status[0] == 0 and b.status[0] == 0
+        assert np.linalg.norm(a.currents - b.currents) <= 1e-7 * np.linalg.norm(b.currents)
