@@ -3589,7 +3589,7 @@ int fnec_server_submit(fnec_server *S, const fnec_antenna *req, const fnec_reque
         info->n_feed_rows = r->n_feed_rows;
         info->n_points = r->n_points;
         info->pad = 0;
-        info->device_bytes = (uint64_t)full;
+        info->device_bytes = (uint64_t)r->bytes;
     }
     if (r->bytes > (int64_t)S->cfg.hbm_budget_bytes) {
         delete r;

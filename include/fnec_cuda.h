@@ -442,7 +442,12 @@ typedef struct {
     uint32_t n_feed_rows;
     uint32_t n_points;
     uint32_t pad;
-    uint64_t device_bytes; /* admission estimate (upper bound) of the footprint */
+    uint64_t device_bytes; /* admission estimate (upper bound) of the footprint.
+                              fnec_request_shape counts the optional scratch of
+                              large mixed systems (S >= 1,536: block inverses,
+                              wide factor steps); fnec_server_submit gives what
+                              the server charges, without that scratch where it
+                              has several lanes or no room for it in its budget */
 } fnec_request_info;
 
 typedef struct {

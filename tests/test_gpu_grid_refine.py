@@ -169,3 +169,16 @@ def test_request_without_the_optional_scratch_leaves_the_others_theirs(acc):
     for a, b in zip(reqs, first + second):
         assert a.status[0] == 0 and b.status[0] == 0
         assert np.linalg.norm(a.currents - b.currents) <= 1e-7 * np.linalg.norm(b.currents)
+
+
+@pytest.mark.parametrize("lanes,short", [(1, 0), (1, 4 << 20), (2, 0)])
+def test_submitted_requests_device_bytes_is_what_admission_charges(acc, lanes, short):
+    w, s, f = bench.mesh_workload(16)
+    ant = acc.Antenna(acc.wires_array(w), acc.sources_array([(7, 1, 1.0)]), [f], 1)
+    with acc.Server(acc.PRECISION_MIXED, lanes=1, hbm_budget_bytes=1 << 30) as srv:
+        full = srv.shape(ant).device_bytes
+    with acc.Server(acc.PRECISION_MIXED, lanes=lanes, hbm_budget_bytes=full - short) as srv:
+        r = srv.wait(srv.submit(ant, copy_out=True))
+        assert r.status[0] == 0
+        assert r.info.device_bytes == srv.stats()["peak_in_flight_bytes"]
+        assert (r.info.device_bytes == full) == (lanes == 1 and short == 0)
