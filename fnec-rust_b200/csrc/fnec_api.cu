@@ -2724,13 +2724,27 @@ int fnec_batch_read_z(fnec_batch *b, uint32_t unit, double *z) {
 
 // Device memory of one call, from the device's stream-ordered pool on the
 // context's stream (cudaMalloc and cudaFree cost a one-call entry most of a
-// millisecond, and stall every stream of the device).
+// millisecond, and stall every stream of the device).  The pool keeps what is
+// freed, so larger blocks, whose copies take longer than that, are the
+// device's own and given back with the call.
+constexpr size_t CALL_POOLED_MAX = 64ull << 20;
 struct CallMemory {
     cudaStream_t st;
     void *p = nullptr;
-    cudaError_t alloc(size_t bytes) { return cudaMallocAsync(&p, bytes, st); }
+    bool pooled = true;
+    cudaError_t alloc(size_t bytes) {
+        pooled = bytes <= CALL_POOLED_MAX;
+        if (!pooled) {
+            const cudaError_t e = cudaMalloc(&p, bytes);
+            if (e != cudaErrorMemoryAllocation) return e;
+            (void)cudaGetLastError();  // the pool may hold the room
+            pooled = true;
+        }
+        return cudaMallocAsync(&p, bytes, st);
+    }
     ~CallMemory() {
-        if (p) cudaFreeAsync(p, st);
+        if (p && pooled) cudaFreeAsync(p, st);
+        else if (p) cudaFree(p);
     }
 };
 
