@@ -2783,7 +2783,8 @@ int fnec_fill_zmatrix(fnec_ctx *ctx, const fnec_zsegment *segments, uint64_t n, 
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(z_out, d_z, sizeof(cx) * n * n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    const cudaError_t done = cudaStreamSynchronize(ctx->stream);  // after an error too: a copy may be in flight
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) return fail(ctx, FNEC_ERR_CUDA, cudaGetErrorString(e));
     return FNEC_OK;
 }
@@ -3041,7 +3042,8 @@ int fnec_near_field(fnec_ctx *ctx, const fnec_gpu_segment *segments, uint64_t n,
     }
     if (e == cudaSuccess && e_out) e = cudaMemcpyAsync(e_out, d_e, sizeof(double) * n_fld, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && h_out) e = cudaMemcpyAsync(h_out, d_h, sizeof(double) * n_fld, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t done = cudaStreamSynchronize(s);  // after an error too: copies may be in flight
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) return fail(ctx, FNEC_ERR_CUDA, cudaGetErrorString(e));
     return FNEC_OK;
 }
