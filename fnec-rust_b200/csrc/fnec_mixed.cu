@@ -1003,6 +1003,13 @@ __global__ void __launch_bounds__(256) k_trailing32(const UnitDesc *__restrict__
 // above it, identity pivots), so the refinement applies it unchanged.
 // A zero or non-finite pivot fails the unit as a singular GEPP panel does.
 
+// 1 / d for a pivot, dn = |d|^2; the roundings written out, so that the
+// panel kernels that form it from the same pivot agree in every bit
+__device__ __forceinline__ float2 herm_pivot_recip(float2 d, float &dn) {
+    dn = __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y));
+    return cf(__fdiv_rn(d.x, dn), __fdiv_rn(-d.y, dn));
+}
+
 // The nb x nb diagonal block at c0, factored by all NT threads: a lane per
 // column, a row (NT = 1024) or four (256) per warp in registers, the pivot
 // row through a double-buffered line of shared memory, one barrier per
@@ -1033,8 +1040,8 @@ __device__ void herm_diag_block(const float2 *A, int s, int c0, int nb, float2 (
     for (int c = 0; c < nb; ++c) {
         __syncthreads();  // row c is complete
         const float2 d = s_row[c & 1][c], p = s_row[c & 1][lane];
-        const float dn = __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y));
-        const float2 dinv = cf(__fdiv_rn(d.x, dn), __fdiv_rn(-d.y, dn));
+        float dn;
+        const float2 dinv = herm_pivot_recip(d, dn);
         if (tid == 0) {
             sDinv[c] = dinv;
             if ((!(dn > 0.f) || !(dn < INFINITY)) && *s_bad == 0) *s_bad = c + 1;
@@ -1242,9 +1249,8 @@ __global__ void __launch_bounds__(HERM_ROWS_CHUNK) k_herm_rows(const UnitDesc *_
     for (int e = tid; e < MNB * MNB; e += HERM_ROWS_CHUNK) sD[e / MNB][e % MNB] = A[(int64_t)(c0 + e / MNB) * s + c0 + e % MNB];
     __syncthreads();
     if (tid < MNB) {  // as herm_diag_block forms them from the same pivots
-        const float2 d = sD[tid][tid];
-        const float dn = d.x * d.x + d.y * d.y;
-        sDinv[tid] = cf(d.x / dn, -d.y / dn);
+        float dn;
+        sDinv[tid] = herm_pivot_recip(sD[tid][tid], dn);
     }
     __syncthreads();
     herm_rows<HERM_ROWS_CHUNK>(A, s, c0, r_begin, min(s, r_begin + HERM_ROWS_CHUNK), sD, sDinv);

@@ -182,3 +182,16 @@ def test_submitted_requests_device_bytes_is_what_admission_charges(acc, lanes, s
         assert r.status[0] == 0
         assert r.info.device_bytes == srv.stats()["peak_in_flight_bytes"]
         assert (r.info.device_bytes == full) == (lanes == 1 and short == 0)
+
+
+@pytest.mark.parametrize("edges", [342, 350, 352])
+def test_split_panel_is_the_one_cta_panel(acc, edges):
+    """S of 1,026 to 1,056: the first panel is one CTA's when the system is
+    alone, and split over many beside a taller one of its size class; the
+    same factor, so the same currents, bit for bit."""
+    w, s, f = bench.mesh_workload(24)
+    ants = [acc.Antenna(acc.wires_array(w[:e]), acc.sources_array([(7, 1, 1.0)]), [f], 1) for e in (edges, 467)]
+    alone = acc.HallenBatch(ants[:1], precision=acc.PRECISION_MIXED).solve()
+    beside = acc.HallenBatch(ants, precision=acc.PRECISION_MIXED).solve()
+    assert alone.status[0] == 0 and beside.status[0] == 0
+    assert np.array_equal(alone.currents[0].view(np.uint64), beside.currents[0].view(np.uint64))
