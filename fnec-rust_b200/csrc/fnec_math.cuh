@@ -74,12 +74,16 @@ FNEC_FN double cx_norm_sqr(cx a) { return D_ADD(D_MUL(a.re, a.re), D_MUL(a.im, a
 //   r  = g + (x - g^2) y/2 with g = x y, the residual exact in an FMA;
 //   z  = y + y (1 - r y), the reciprocal of r;
 //   a/r = q + (a - q r) z with q = a z.
-// The last two corrections are Markstein's (Computation of elementary
-// functions on the IBM RISC System/6000 processor, 1990): the value before
-// the final rounding is within 2^-103 of exact, relative, and the result is
-// the rounded one.  Domain: x normal in [2^-100, 2^100) and quotients whose
-// residual stays normal (a zero, or |a| above 2^-800); callers fall back to
-// the general operations outside.
+// The last corrections are Markstein's (Computation of elementary functions
+// on the IBM RISC System/6000 processor, 1990): with z the rounded reciprocal
+// of r and q within an ulp, a/r comes out rounded, and so does z itself unless
+// r's mantissa is all ones.  The root's value before its final rounding is
+// within about 2^-103 of exact, relative.  That bound alone does not settle
+// every root (they come as near as about 2^-107 to the middle of two doubles):
+// tests/test_gpu_exact_division.py constructs roots and quotients from 2^-97
+// to 2^-104 of a middle and finds no wrong bit on the device.  Domain: x normal
+// in [2^-100, 2^100) and quotients whose residual stays normal (a zero, or |a|
+// above 2^-800); callers fall back to the general operations outside.
 // ---------------------------------------------------------------------------
 struct SqrtRecip {
     double r, z;  // sqrt(x), 1/sqrt(x) rounded from r

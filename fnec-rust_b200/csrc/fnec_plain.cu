@@ -2098,3 +2098,61 @@ int selftest_grid_timeout(int32_t device, int32_t ctas, int32_t absent, uint64_t
     return rc;
 }
 }  // namespace fnec
+
+// ---------------------------------------------------------------------------
+// Self-test of the shortened divisions and square root (fnec_test_exact_
+// division): every one against the IEEE operation, bit for bit, inside the
+// range that its callers guard.
+// ---------------------------------------------------------------------------
+namespace fnec {
+__global__ void k_test_exact_division(const double *av, const double *xv, int n, int32_t *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double a = av[i], x = xv[i];
+    auto differ = [](double p, double q) { return __double_as_longlong(p) != __double_as_longlong(q); };
+    auto exponent_within = [](double v, int e) {  // 2^-e <= |v| < 2^e
+        const int k = (int)((uint32_t)(fnec_libm::lm_hi(v) & 0x7fffffffu) >> 20) - 1023;
+        return k >= -e && k < e;
+    };
+    int bad = 0;
+    if (sqrt_recip_domain(x)) {
+        const SqrtRecip sr = sqrt_recip(x);
+        if (differ(sr.r, D_SQRT(x))) bad |= 1;
+        if ((a == 0.0 || exponent_within(a, 400)) && differ(div_by(a, sr), D_DIV(a, sr.r))) bad |= 2;
+    }
+    if (x > 0.0 && exponent_within(x, 400) && (uint32_t)fnec_libm::lm_bits(x) != 0xffffffffu) {
+        const double z = recip_rn(x);
+        if (differ(z, D_DIV(1.0, x))) bad |= 4;
+        if ((a == 0.0 || exponent_within(a, 400)) && differ(div_by(a, {x, z}), D_DIV(a, x))) bad |= 8;
+    }
+    const cx num = cx_make(a, x), den = cx_make(x, -a);
+    const double ns = D_ADD(D_MUL(den.re, den.re), D_MUL(den.im, den.im));
+    const cx p = cp_div(num, den, ns, recip_rn(ns)), q = cx_div(num, den);
+    if (differ(p.re, q.re) || differ(p.im, q.im)) bad |= 16;
+    out[i] = bad;
+}
+}  // namespace fnec
+
+extern "C" int fnec_test_exact_division(const double *a, const double *x, uint64_t n, int32_t *out) {
+    if (n && (!a || !x || !out)) return FNEC_ERR_BAD_ARG;
+    if (n > ((uint64_t)1 << 24)) return FNEC_ERR_TOO_LARGE;
+    for (uint64_t i = 0; i < n; ++i)
+        if (!std::isfinite(a[i]) || !std::isfinite(x[i])) return FNEC_ERR_BAD_ARG;
+    if (n == 0) return FNEC_OK;
+    unsigned char *d = nullptr;
+    if (cudaMalloc(&d, (2 * sizeof(double) + sizeof(int32_t)) * n) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return FNEC_ERR_OUT_OF_MEMORY;
+    }
+    double *da = reinterpret_cast<double *>(d), *dx = da + n;
+    int32_t *dout = reinterpret_cast<int32_t *>(dx + n);
+    cudaError_t e = cudaMemcpy(da, a, sizeof(double) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(dx, x, sizeof(double) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        fnec::k_test_exact_division<<<(unsigned)((n + 255) / 256), 256>>>(da, dx, (int)n, dout);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, dout, sizeof(int32_t) * n, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? FNEC_OK : FNEC_ERR_CUDA;
+}

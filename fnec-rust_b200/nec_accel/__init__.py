@@ -201,6 +201,7 @@ SIGNATURES = {
     "fnec_test_limit_refinement_ctas": (ctypes.c_int, [_I32]),
     "fnec_test_fill_sincospi": (ctypes.c_int, [_P, _U64, _P, _P]),
     "fnec_test_fill_rsqrt": (ctypes.c_int, [_P, _U64, _P]),
+    "fnec_test_exact_division": (ctypes.c_int, [_P, _P, _U64, _P]),
     "fnec_host_cache_release": (ctypes.c_int, [_P]),
     "fnec_device_cache_release": (ctypes.c_int, [_P, _P]),
     "fnec_batch_create": (ctypes.c_int, [_P, _P, _U32, _I32, _P]),
@@ -663,6 +664,21 @@ def test_fill_rsqrt(x):
     rc = lib().fnec_test_fill_rsqrt(_ptr(x), len(x), _ptr(out))
     if rc != OK:
         raise AccelError(rc, "test_fill_rsqrt")
+    return out
+
+
+def test_exact_division(a, x):
+    """Test hook: the plain form's square root and divisions on the current
+    device against the IEEE operations; per pair the bits that
+    fnec_test_exact_division names."""
+    a = np.ascontiguousarray(a, dtype=np.float64)
+    x = np.ascontiguousarray(x, dtype=np.float64)
+    if a.shape != x.shape:
+        raise ValueError("a and x differ in shape")
+    out = np.empty(a.shape, np.int32)
+    rc = lib().fnec_test_exact_division(_ptr(a), _ptr(x), a.size, _ptr(out))
+    if rc != OK:
+        raise AccelError(rc, "test_exact_division")
     return out
 
 

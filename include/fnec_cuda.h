@@ -569,6 +569,12 @@ int fnec_test_fill_sincospi(const double *x, uint64_t n, double *sin_out, double
  * Newton steps), run on the current device for n <= 2^20 normal, finite,
  * positive arguments (test use; allocates its own device memory). */
 int fnec_test_fill_rsqrt(const double *x, uint64_t n, double *out);
+/* The plain form's square root and divisions through shared reciprocals, run
+ * on the current device for n <= 2^24 finite pairs against the IEEE
+ * operations (test use).  out[i]: 1 sqrt(x), 2 a / sqrt(x), 4 1 / x, 8 a / x,
+ * 16 the complex quotient (a + ix) / (x - ia) differ in a bit; a pair outside
+ * a form's guarded range is not compared in it. */
+int fnec_test_exact_division(const double *a, const double *x, uint64_t n, int32_t *out);
 
 /* Radiation pattern that allocates no device memory.  No counterpart in
  * the reference: it serves callers that cannot call cudaMalloc -- a host
