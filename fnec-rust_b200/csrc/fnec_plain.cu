@@ -289,7 +289,7 @@ struct FillTile {
     double tab[4][112];     // the sin/cos table by part
     double rs[8][3][16];    // source points (node, axis, source)
     double om[3][16], od[3][16], sd[3][16];
-    double half[16], a2[16], rad[16], self_log[16];
+    double half[16], a2[16], self_log[16];
 };
 
 struct LmSharedTable {
@@ -334,7 +334,6 @@ __device__ __forceinline__ void fill_exact_tile(FillTile &sh, const DevSeg *__re
 #pragma unroll
             for (int c = 0; c < 3; ++c) sh.sd[c][tid] = s.dir[c];
             sh.half[tid] = half;
-            sh.rad[tid] = s.rad;
             sh.a2[tid] = D_MUL(s.rad, s.rad);
             sh.self_log[tid] = s.self_log;
         }
@@ -602,7 +601,8 @@ __device__ __forceinline__ void piv_better(double &bv, int &bi, double v, int i)
 }
 
 __global__ void __launch_bounds__(256) k_panel(const UnitDesc *__restrict__ units, int c0,
-                                               cx *abuf, int32_t *piv_buf, int32_t *status, int skip_m, const int32_t *__restrict__ order, int base) {
+                                               cx *abuf, int32_t *piv_buf, int32_t *status,
+                                               const int32_t *__restrict__ order, int base) {
     __shared__ double s_v[8];
     __shared__ int s_i[8];
     __shared__ int s_p;
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(256) k_panel(const UnitDesc *__restrict__ unit
     int ui = order[base + blockIdx.x];
     UnitDesc u = units[ui];
     int s = u.s;
-    if (c0 >= s || s - c0 > skip_m || status[ui] != 0) return;  // skip_m: taller panels go grid-wide
+    if (c0 >= s || status[ui] != 0) return;
     int w1 = s + 1;
     cx *A = abuf + u.a_off;
     int32_t *piv = piv_buf + u.piv_off;
@@ -1935,7 +1935,7 @@ uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const Gri
                        cudaSuccess;
                 if (!done) (void)cudaGetLastError();  // not co-resident after all
             }
-            if (!done) k_panel<<<n_thr, 256, 0, st>>>(units, c0, A, piv, status, INT_MAX, ord, 0);
+            if (!done) k_panel<<<n_thr, 256, 0, st>>>(units, c0, A, piv, status, ord, 0);
             ++L;
         }
         step_classes(gp, c0, n_thr, cls);
