@@ -60,9 +60,9 @@ struct DevAlloc {
     }
 };
 
-// Units whose panels are too tall for one CTA's shared memory (mixed) or one
-// cluster's registers (plain, above 3,072 rows) are factored by the grid-wide
-// panel kernel (fnec_grid.cuh).  Built once per batch.
+// Units whose panels are too tall for one CTA's shared memory (mixed) or for
+// the largest cluster of CTAs (plain, above 3,072 rows) are factored by the
+// grid-wide panel kernel (fnec_grid.cuh).  Built once per batch.
 struct GridPlan {
     int32_t *d_order = nullptr;  // unit indices, s descending
     std::vector<int> s_desc;     // their s (host copy)

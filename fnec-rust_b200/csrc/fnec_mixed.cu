@@ -646,8 +646,12 @@ constexpr int TC_TRAIL_MIN_M = 192;
 // Measured, factor phase, 32 against 128 columns: 46 x 46 mesh (S = 12,972)
 // 99.5 -> 43.1 ms (the trailing kernels 87.6 -> 28.6), 30 x 30 (S = 5580)
 // 14.2 -> 10.7, 20 x 20 (2520) 4.24 = 4.24, 16 x 16 (1632) 2.89 < 3.02 ms:
-// hence the bound on S.  The 3xTF32 products leave the refinement's final
-// residual at or below the FP32 tiles' (S = 1632 to 12,972: 0.4 to 0.7 of it).
+// hence the bound on S.  The 3xTF32 products are summed over 128 columns in
+// TMEM and A22 is rounded once for them, where the 32-column FP32 tiles round
+// it at every product.  Factor error against 64 bits, |A - L U| of the same
+// normal matrix, 128 columns over 32: meshes of 23 to 46 cells (S = 3312 to
+// 12,972), Frobenius 0.11 to 0.043, largest |E_ij| / sqrt(a_ii a_jj) 0.33 to
+// 0.06, its rms 0.26 to 0.064; the refinement's final residual 0.4 to 0.7.
 constexpr int WIDE = 128;
 constexpr int WIDE_MIN_S = 3072;  // and at most TC_WIDE_MAX_UNITS such units
 constexpr int FU_THREADS = 256;
@@ -2642,8 +2646,6 @@ __global__ void __launch_bounds__(256, 2) k_gmres_cluster(
     gmres_grid_body(c, u, mus, ui, xbuf, W, vbuf + mu.v_off);
 }
 
-// The row permutation of the factor: perm[i] = source row of row i after
-// the swaps piv[0..s) (applied in order, in shared memory when it fits).
 // ---------------------------------------------------------------------------
 // Inverses, in FP64, of the FP32 factor's GI-row diagonal blocks of one
 // system, for the grid-wide refinement: inv[(block * 2 + which) * GI * GI],
@@ -2742,6 +2744,8 @@ __global__ void __launch_bounds__(256) k_gi_double(const UnitDesc *__restrict__ 
     }
 }
 
+// The row permutation of the factor: perm[i] = source row of row i after
+// the swaps piv[0..s) (applied in order, in shared memory when it fits).
 __global__ void k_perm_from_piv(const UnitDesc *__restrict__ units, int ui, const int32_t *__restrict__ pivbuf,
                                 int32_t *perm, int staged) {
     extern __shared__ int32_t s_perm_dyn[];
@@ -3145,8 +3149,9 @@ void free_mixed(MixedWork &w, const DevAlloc &dev) {
 
 // The FP64 GMRES refinement of every solve on the stored FP32 factor (the
 // last part of run_mixed; also a resident system's re-solve with new
-// right-hand sides, where the factor and its block inverses are reused:
-// fresh_factor false).
+// right-hand sides, where the factor and its 32-row block inverses are
+// reused: fresh_factor false).  The grid-wide refinement's 256-row inverses
+// share one buffer and are formed for each solve.
 uint64_t refine_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDesc *d_solves, int ns,
                       const AntDesc *d_ants, const int32_t *ibuf, const DevConRow *crows, const cx *z, const cx *rhs,
                       const double *cosv, cx *x, int32_t *piv, int32_t *status, int max_s, MixedMarks &marks,
@@ -3324,7 +3329,7 @@ uint64_t run_mixed(MixedWork &mw, const UnitDesc *d_units, int nu, const UnitDes
         while (i_unit > 0 && gp.s_desc[i_unit - 1] <= fu_max_s(gp.unit_factor)) --i_unit;
     const bool unit_launch = i_unit < nu_all;
     // the tallest units of the Hermitian factor take wide steps, ahead of
-    // the others (tensor_trailing 1 and 2 keep 32-column steps for all)
+    // the others (tensor_trailing 1 and 2 keep 32-column steps for all; 2 in FP32 SIMT tiles)
     const int n_wide = herm && mw.wide && !mw.use_tc_trail && !mw.two_step ? std::min(mw.wide_n, i_unit) : 0;
     int G = std::max(1, std::min(gp.factor_streams, MixedWork::MAX_FACTOR_STREAMS) - (unit_launch ? 1 : 0));
     if (!mw.fmade || i_unit - n_wide < 2 * G) G = 1;

@@ -1825,9 +1825,10 @@ size_t grid_xchg_bytes() { return sizeof(PanelXchg<cx>) * GRID_PANEL_MAX_UNITS; 
 size_t grid_sync_bytes(int steps) { return sizeof(GridSync) * GRID_PANEL_MAX_UNITS * (size_t)(steps > 0 ? steps : 1); }
 
 // Chooses how the panel at column c0 is factored.  Units whose panel
-// (s - c0 rows) exceeds one CTA's shared memory (thr_rows) go to the
-// grid-wide kernel when they are few enough to be co-resident; the rest use
-// the one-CTA shared-memory kernel.  Returns the number of grid units
+// (s - c0 rows) exceeds thr_rows (plain: the largest cluster's rows; mixed:
+// one CTA's shared memory) go to the grid-wide kernel when they are few enough
+// to be co-resident; the rest take the form's own kernel for shorter panels.
+// Returns the number of grid units
 // (0: none; -1: not possible, every unit takes the one-CTA global kernel)
 // and the CTAs per grid unit and their shared memory.
 int plan_grid_panel(const GridPlan &gp, int c0, int thr_rows, int pnb, size_t elem, const void *kernel,

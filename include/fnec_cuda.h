@@ -691,7 +691,7 @@ int fnec_batch_resolve(fnec_batch *b);
  * tolerance under every schedule. */
 typedef struct {
     int32_t grid_panels;   /* 1: panels too tall for one CTA's shared memory (mixed)
-                              or one cluster's registers (plain, above 3,072 rows)
+                              or the largest cluster (plain, above 3,072 rows)
                               are factored grid-wide (cooperative launch); 0: one
                               CTA from global memory                              */
     int32_t class_shift;   /* panel and trailing launches group units whose
@@ -720,16 +720,18 @@ typedef struct {
                               for the Hermitian factor only the tiles on and
                               below the diagonal); 0 all as FP32 SIMT tiles, one
                               pass per step, but up to 16 Hermitian systems
-                              of S >= 3072 in 128-column tcgen05 steps; 2 (GEPP only) SIMT tiles once per
-                              two steps (the first step updates only the next
-                              panel's columns)                                   */
+                              of S >= 3072 (where there is room for the operands)
+                              in 128-column tcgen05 steps; 2 FP32 SIMT tiles for
+                              every system: with GEPP once per two steps (the
+                              first step updates only the next panel's columns),
+                              with the Hermitian factor one pass per step       */
     int32_t gmres_ctas_per_sm;/* mixed: 3 or 4 refinement CTAs per SM (the
                               register budget of the one-CTA-per-solve kernel)    */
     int32_t factor_pivoting;/* mixed: 0 the FP32 factor of the Hermitian normal
                               equations without row exchanges (lower-triangle
                               trailing updates, U12 mirrored from L21); 1 GEPP
                               with partial pivoting (row exchanges and U12
-                              solves; tensor_trailing 2 applies to it only)     */
+                              solves)                                           */
 } fnec_schedule;
 
 /* Graph state of a batch (fnec_batch_graph_state). */
