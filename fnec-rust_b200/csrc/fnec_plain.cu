@@ -21,7 +21,7 @@
 //   k_panel            linear.rs:1343-1370     the same from global memory, one CTA per unit
 //   k_panel_grid       linear.rs:1343-1370     NB columns of a panel above 3,072 rows, many CTAs
 //   k_swap_u12         linear.rs:1358-1369     deferred swaps + U block row
-//   k_trailing         linear.rs:1362-1369     A22 -= L21 U12, 32x32 tiles
+//   k_trailing         linear.rs:1362-1369     A22 -= L21 U12, 32x32 or 64x64 tiles
 //   k_backsub          linear.rs:1372-1381     one CTA per unit: a chain warp, two product warps
 //   k_feedpoints       solve_session.rs:846-947
 #include <algorithm>
@@ -1126,17 +1126,23 @@ constexpr size_t SU_SMEM = sizeof(cx) * (2 * NB * SU_LD + NB * (NB + 1));
 
 // A22 -= L21 * U12 with per-element in-order accumulation over the panel.
 // grid.x = tiles of TT x TT over the trailing block, grid.y = unit.
-// 32 wide, as the Gram's tiles, for their raggedness and the number of CTAs;
-// the panel blocks stage by cp.async beside the tile's own loads.  Measured,
-// factor phase, against 64 x 64 tiles staged first: one N = 255 system 0.65
-// -> 0.57 ms, 512 random antennas 10.4 -> 9.4, 20 x 20 mesh 11.4 -> 10.9,
-// 30 x 30 (S = 5580) 55.0 -> 55.4.
-constexpr int TT = 32;
+// The panel blocks stage by cp.async beside the tile's own loads.  32 wide, as
+// the Gram's tiles, for their raggedness and the number of CTAs: factor phase
+// against 64 x 64 tiles staged first, one N = 255 system 0.65 -> 0.57 ms, 512
+// random antennas 10.4 -> 9.4, 20 x 20 mesh 11.4 -> 10.9.  64 wide from
+// TRAILING_WIDE_ROWS on, where neither counts and each entry of a staged block
+// serves four products instead of two: 46 x 46 mesh (S = 12,972) 448 -> 426 ms,
+// 40 x 40 (9840) 214 -> 205, 30 x 30 (5580) 55.1 -> 54.0, 24 x 24 (3600) 21.28
+// -> 21.22; the same from 1024 or 3072 rows on, and 20 x 20 (2520) 10.83 = 10.85
+// from 2048 on but 10.96 from 1024.
+constexpr int TRAILING_WIDE_ROWS = 2048;
+template <int TT>
 __global__ void __launch_bounds__(256) k_trailing(const UnitDesc *__restrict__ units, int c0,
                                                   cx *abuf, const int32_t *__restrict__ status, const int32_t *__restrict__ order, int base) {
     constexpr int P = TT / 16;
-    __shared__ cx s_l[TT][NB + 1];
-    __shared__ cx s_u[NB][TT];
+    extern __shared__ cx s_tt[];
+    cx(*s_l)[NB + 1] = reinterpret_cast<cx(*)[NB + 1]>(s_tt);
+    cx(*s_u)[TT] = reinterpret_cast<cx(*)[TT]>(s_tt + TT * (NB + 1));
     int ui = order[base + blockIdx.y];
     UnitDesc u = units[ui];
     int s = u.s;
@@ -1170,7 +1176,7 @@ __global__ void __launch_bounds__(256) k_trailing(const UnitDesc *__restrict__ u
         }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-#pragma unroll 4
+#pragma unroll (TT == 32 ? 4 : 1)
     for (int q = 0; q < NB; ++q) {
         cx lv[P], uv[P];
 #pragma unroll
@@ -1189,6 +1195,14 @@ __global__ void __launch_bounds__(256) k_trailing(const UnitDesc *__restrict__ u
             int R = R0 + ty + 16 * a, K = K0 + tx + 16 * b;
             if (R < s && K <= s) A[(int64_t)R * w1 + K] = acc[a][b];
         }
+}
+template <int TT>
+static void launch_trailing(const UnitDesc *units, int n, int rows, int cols, int c0, cx *A, int32_t *status,
+                            const int32_t *order, int base, cudaStream_t st) {
+    constexpr size_t smem = sizeof(cx) * (TT * (NB + 1) + NB * TT);
+    set_smem_limit_once(k_trailing<TT>, (int)smem);
+    dim3 g(((rows + TT - 1) / TT) * ((cols + TT - 1) / TT), n);
+    k_trailing<TT><<<g, 256, smem, st>>>(units, c0, A, status, order, base);
 }
 
 // Back substitution x_i = (b_i - sum_{j>i} a_ij x_j) / a_ii, j ascending.
@@ -1955,9 +1969,8 @@ uint64_t launch_factor_exact(const UnitDesc *units, int nu, int max_s, const Gri
             ++L;
             int rows = m - NB;
             if (rows > 0) {
-                int t = ((rows + TT - 1) / TT) * ((rest + TT - 1) / TT);
-                dim3 g2(t, c.i1 - c.i0);
-                k_trailing<<<g2, 256, 0, st>>>(units, c0, A, status, ord, c.i0);
+                const auto trailing = rows >= TRAILING_WIDE_ROWS ? launch_trailing<64> : launch_trailing<32>;
+                trailing(units, c.i1 - c.i0, rows, rest, c0, A, status, ord, c.i0, st);
                 ++L;
             }
         }
