@@ -3181,7 +3181,7 @@ int64_t request_bytes(const HostAnt &h, int precision, bool large = true) {
     int64_t b = 0;
     b += 16 * n * n * f;                                   // Z
     b += 160 * n + 256 * w + 64 * rows + 4 * n_int;        // geometry, tables, coverage maps
-    b += n * n / 16 + 64 * ((n + 63) / 64) * ((n + 64) / 64);  // fill and Gram tile lists
+    b += ((n + 15) * (n + 15) / 16 + 64 * ((n + 63) / 64) * ((n + 64) / 64)) * f;  // fill and Gram tile lists
     b += 16 * n * f * r;                                   // compact currents for pinned reads
     b += (16 * s + 16 * n + 8 * n + 64) * f * r;           // x, rhs, cos, feeds
     if (h.planewave) b += 8 * n * f + 8 * f * r + 80 * r + 16 * n + 8 * n * n * f;  // sin column, peaks,

@@ -195,3 +195,18 @@ def test_split_panel_is_the_one_cta_panel(acc, edges):
     beside = acc.HallenBatch(ants, precision=acc.PRECISION_MIXED).solve()
     assert alone.status[0] == 0 and beside.status[0] == 0
     assert np.array_equal(alone.currents[0].view(np.uint64), beside.currents[0].view(np.uint64))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("wires,segments,freqs", [(6, 101, 100), (1, 17, 300), (2, 801, 8)])
+def test_footprint_of_many_frequencies_bounds_the_batch(acc, precision, wires, segments, freqs):
+    """The fill's and the Gram's tile lists hold an entry per tile of every
+    frequency's system: the admission estimate counts them all."""
+    w = [(t + 1, segments, (2.0 * t, 0.0, -5.0), (2.0 * t, 0.0, 5.0), 1e-3) for t in range(wires)]
+    f = [14.0e6 + 1e3 * k for k in range(freqs)]
+    ant = acc.Antenna(acc.wires_array(w), acc.sources_array([(1, segments // 2, 1.0)]), f, 0)
+    with acc.Server(precision, lanes=1, hbm_budget_bytes=1 << 30) as srv:
+        est = srv.shape(ant).device_bytes
+    b = acc.HallenBatch([ant], precision=precision)
+    assert b.info.device_bytes <= est, (b.info.device_bytes, est)
+    b.close()
