@@ -652,6 +652,9 @@ constexpr int TC_TRAIL_MIN_M = 192;
 // normal matrix, 128 columns over 32: meshes of 23 to 46 cells (S = 3312 to
 // 12,972), Frobenius 0.11 to 0.043, largest |E_ij| / sqrt(a_ii a_jj) 0.33 to
 // 0.06, its rms 0.26 to 0.064; the refinement's final residual 0.4 to 0.7.
+// Wire arrays, one long wire and random antennas of S = 3202 to 4080: 0.03 to
+// 0.53, 0.04 to 0.22 and 0.03 to 0.06 (there the residual at the stop, below
+// its tolerance either way, is the smaller one of either factor).
 constexpr int WIDE = 128;
 constexpr int WIDE_MIN_S = 3072;  // and at most TC_WIDE_MAX_UNITS such units
 constexpr int FU_THREADS = 256;
