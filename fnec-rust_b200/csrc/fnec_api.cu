@@ -2725,9 +2725,10 @@ int fnec_batch_read_z(fnec_batch *b, uint32_t unit, double *z) {
 // Device memory of one call, from the device's stream-ordered pool on the
 // context's stream (cudaMalloc and cudaFree cost a one-call entry most of a
 // millisecond, and stall every stream of the device).  The pool keeps what is
-// freed, so larger blocks, whose copies take longer than that, are the
-// device's own and given back with the call.
-constexpr size_t CALL_POOLED_MAX = 64ull << 20;
+// freed, so large blocks are the device's own and given back with the call:
+// above 256 MB that millisecond is under 2 % of it (fill_zmatrix, 70 MB: 16.8
+// ms from the pool, 17.8 without).
+constexpr size_t CALL_POOLED_MAX = 256ull << 20;
 struct CallMemory {
     cudaStream_t st;
     void *p = nullptr;

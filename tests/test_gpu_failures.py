@@ -223,9 +223,9 @@ def test_optional_scratch_is_allocated_last(acc):
 
 
 def test_large_single_calls_keep_no_device_memory(acc):
-    """fill_zmatrix and near_field with more than 64 MB on the device: the
+    """fill_zmatrix and near_field with more than 256 MB on the device: the
     call gives it back; the pool keeps smaller blocks only."""
-    n, p = 2100, 600_000
+    n, p = 4200, 2_400_000
     segs = O.build_geometry(O.wires_array([(1, n, (0.0, 0.0, -50.0), (0.0, 0.0, 50.0), 1e-3)]))
     pts = np.random.default_rng(0).uniform(1.0, 9.0, (p, 3))
     small = np.ascontiguousarray(segs[:64])
@@ -233,8 +233,8 @@ def test_large_single_calls_keep_no_device_memory(acc):
     acc.device_cache_release()
     z = acc.fill_zmatrix(acc.zsegments_from(segs), 14.2e6, 0)
     assert np.array_equal(z[:64, :64], ref)
-    assert acc.device_cache_release() < 64 << 20
+    assert acc.device_cache_release() < 128 << 20
     e, h = acc.near_field(acc.gpu_segments_from(small), np.ones(64, complex), 14.2e6, pts)
-    assert acc.device_cache_release() < 64 << 20
+    assert acc.device_cache_release() < 128 << 20
     e0, h0 = acc.near_field(acc.gpu_segments_from(small), np.ones(64, complex), 14.2e6, pts[-40:])
     assert np.array_equal(e[-40:], e0) and np.array_equal(h[-40:], h0)
